@@ -20,7 +20,9 @@
 // in magnitude -- (L+1) products of at most 128 * 64 per k, or 128^2 for
 // L = 0 -- so its FP32 accumulation in TMEM is exact; levels 6 and 7 carry
 // weights 2^-56 and 2^-63 and their FP32 rounding is far below FP64 rounding.
-// Longer K runs in passes of 512 that accumulate into C.
+// Longer K runs in passes of 512 whose integer level sums add up exactly in
+// registers (one launch and one rounding per 2048 of K); chunks of 2048
+// accumulate into C.
 //
 // Tensor-core layout.  Output tile 128 x 64.  The eight digit planes of the
 // column operand are stacked along N in shared memory (plane t = rows
@@ -29,17 +31,26 @@
 // s + t.  TMEM holds the eight level blocks (512 columns); an MMA wider than
 // 256 columns is issued as two, reusing A through the collector buffer.
 //
-// Recombination (epilogue, per element): the exact levels 0..5 are combined
-// in a 64-bit integer, levels 6..7 in FP32 and rounded in at 2^-3 of a level-5
-// unit; the single rounding to FP64 is that of the integer conversion, and
-// the scale 2^(e_m + f_n) is applied to the exponent field.
+// Recombination (epilogue, per element): the exact levels 0..5 in a 64-bit
+// integer and levels 6..7 in FP32, summed over the passes; one rounding to
+// FP64, in integer instructions.  TMEM holds one set of level blocks, so the
+// MMAs wait while a pass's sums are read: that part is only conversion and
+// integer multiply-adds (about 25 instructions per element, eight warps), and
+// the normalisation, scaling and stores run under the next tile's MMAs.
 //
-// CTA = 6 warps, persistent, one CTA per SM, output tiles assigned round
+// CTA = 10 warps, persistent, one CTA per SM, output tiles assigned round
 // robin: warp 0 bulk-copies the digit planes (two stages of 96 KB: 8 row
 // planes of 128 x 32 and 8 column planes of 64 x 32, each a 64-byte-swizzled
-// shared-memory image), warp 1 owns TMEM and issues the MMAs, warps 2..5
+// shared-memory image), warp 1 owns TMEM and issues the MMAs, warps 2..9
 // read TMEM and write C.  Every wait is bounded.
+//
+// Bound by the tensor pipe: 36 BF16 products per FP64 product, 53 TFLOP/s at
+// the measured cuBLAS BF16 rate.  Measured, kernel alone: 4096 x 32768 x 2048
+// 10.35 ms (53.1 TFLOP/s; 17.5 ms with four epilogue warps that converted
+// through the FP64 pipe before they released TMEM), 4096 x 4096 x 512 0.376 ms
+// (0.526), 1520^3 0.160 ms (0.266).
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "dgemm_tc.h"
@@ -54,12 +65,16 @@ constexpr int TM = 128;                   // output tile rows
 constexpr int TN = 64;                    // output tile columns
 constexpr int DKB = 32;                   // K per stage: 64-byte tile rows
 constexpr int KPASS = 512;                // K per pass (exact levels 0..5)
+constexpr int KCHUNK = 2048;              // K per launch (digit planes in the workspace)
+constexpr int PASS_KB = KPASS / DKB;
 constexpr int A_PLANE = TM * DKB * 2;     // 8 KB
 constexpr int B_PLANE = TN * DKB * 2;     // 4 KB
 constexpr int A_BYTES = DS * A_PLANE;     // 64 KB
 constexpr int STAGE = A_BYTES + DS * B_PLANE;  // 96 KB
 constexpr int NSTAGE = 2;
-constexpr int NTHREADS = 192;
+constexpr int EWARPS = 8;                 // epilogue warps: two per TMEM lane quarter
+constexpr int ECOLS = TN / (EWARPS / 4);  // columns of an epilogue warp
+constexpr int NTHREADS = 64 + 32 * EWARPS;
 constexpr uint32_t SW64 = 4;              // descriptor layout type: 64-byte swizzle
 constexpr uint32_t TMEM_COLS = 512;
 
@@ -74,110 +89,166 @@ __device__ __forceinline__ long long view_row(const MatView& v, long long r) {
 }
 
 // ---------------------------------------------------------------- slicing
-// e[r] = (largest biased exponent of row r over k0 <= k < k0 + kn) - 1022,
-// so |x| < 2^e[r]; rows without a normal value get 0 (all digits zero).
-template <bool WARP_ROW>
-__global__ void __launch_bounds__(256) row_exponent_kernel(MatView v, int rows, int rows_pad,
-                                                           int k0, int kn, int* __restrict__ e) {
-  if (WARP_ROW) {  // one warp per row, k contiguous
-    const int lane = threadIdx.x & 31;
-    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows_pad;
-         r += ((long long)gridDim.x * blockDim.x) >> 5) {
-      int em = 0;
-      if (r < rows) {
-        const double* p = v.p + view_row(v, r) + (long long)k0 * v.ks;
-        for (int k = lane; k < kn; k += 32)
-          em = max(em, (int)((__double_as_longlong(p[(long long)k * v.ks]) >> 52) & 0x7FF));
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
-      if (lane == 0) e[r] = em > 0 ? em - 1022 : 0;
-    }
-  } else {  // one thread per row (coalesced when consecutive rows are adjacent)
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows_pad;
-         r += (long long)gridDim.x * blockDim.x) {
-      int em = 0;
-      if (r < rows) {
-        const double* p = v.p + view_row(v, r) + (long long)k0 * v.ks;
-        for (int k = 0; k < kn; ++k)
-          em = max(em, (int)((__double_as_longlong(p[(long long)k * v.ks]) >> 52) & 0x7FF));
-      }
-      e[r] = em > 0 ? em - 1022 : 0;
-    }
-  }
+// The largest biased exponent of each row, em[r] (0 for a row without a normal
+// value: all digits zero).  |x| < 2^(em - 1022) over the row.
+__device__ __forceinline__ int row_scale(int em) { return em > 0 ? em - 1022 : 0; }
+__device__ __forceinline__ int biased_exponent(double x) {
+  return (__double2hiint(x) >> 20) & 0x7FF;
 }
 
-// The eight BF16 digit bit patterns of x / 2^er, most significant first.
-__device__ __forceinline__ void digits_of(double x, int er, uint32_t (&d)[DS]) {
-  const long long bits = __double_as_longlong(x);
-  const int E = (int)((bits >> 52) & 0x7FF);
-  const uint32_t sgn = bits < 0 ? 0x8000u : 0u;
+// The eight digits of x / 2^er as FP32 integers, most significant first.
+__device__ __forceinline__ void digits_of(double x, int er, float (&d)[DS]) {
+  const int hi = __double2hiint(x);
+  const int E = (hi >> 20) & 0x7FF;
   unsigned long long H = 0;  // round(|x| 2^(56 - er)) <= 2^56
   if (E > 0) {
-    const unsigned long long m = ((unsigned long long)bits & ((1ull << 52) - 1)) | (1ull << 52);
+    const unsigned long long m =
+        ((unsigned long long)((hi & 0xFFFFF) | 0x100000) << 32) | (uint32_t)__double2loint(x);
     const int t = E - 1019 - er;  // <= 3
     if (t >= 0) H = m << t;
     else if (t > -54) H = (m + (1ull << (-t - 1))) >> (-t);
   }
-  // balanced digits: add 64 at each of the seven low base-128 positions
+  // balanced digits: add 64 at each of the seven low base-128 positions, then
+  // digit = (7-bit field) - 64; the sign of x in the one FMA that converts a
+  // field (bits of 2^23 + field) to the signed digit, exactly
   constexpr unsigned long long BIAS = 0x40ull | (0x40ull << 7) | (0x40ull << 14) |
                                       (0x40ull << 21) | (0x40ull << 28) | (0x40ull << 35) |
                                       (0x40ull << 42);
   const unsigned long long Hb = H + BIAS;
+  const float sg = hi < 0 ? -1.f : 1.f;
+  const float c64 = -8388672.0f * sg, c0 = -8388608.0f * sg;
+  const uint32_t w0 = (uint32_t)Hb, w1 = (uint32_t)(Hb >> 28), w2 = (uint32_t)(Hb >> 49);
 #pragma unroll
   for (int p = 0; p < 7; ++p) {
-    const uint32_t u = (uint32_t)(Hb >> (7 * p)) & 127u;
-    const float f = __int_as_float(0x4B000000 | (int)u) - 8388672.0f;  // u - 64, exact
-    d[DS - 1 - p] = (__float_as_uint(f) >> 16) ^ sgn;
+    const uint32_t u = ((p < 4 ? w0 >> (7 * p) : w1 >> (7 * (p - 4))) & 127u) | 0x4B000000u;
+    d[DS - 1 - p] = fmaf(__uint_as_float(u), sg, c64);
   }
-  const uint32_t top = (uint32_t)(Hb >> 49);  // 0 .. 128
-  const float f = __int_as_float(0x4B000000 | (int)top) - 8388608.0f;
-  d[0] = (__float_as_uint(f) >> 16) ^ sgn;
+  d[0] = fmaf(__uint_as_float(w2 | 0x4B000000u), sg, c0);  // 0 .. 128
+}
+// Two small integers (exact in BF16) packed as BF16, the first in the low half.
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
-// Digit planes of rows [0, rows_pad) over k0 <= k < k0 + kn (zero beyond rows
-// and kn), tile images [rt][kb][s] of TR x 32.  One thread per (row, 8 k).
-// ROW_FAST: consecutive threads take consecutive rows (for views whose rows
-// are adjacent in memory); else consecutive k chunks of one row.
-template <int TR, bool ROW_FAST>
-__global__ void __launch_bounds__(256) slice_digits_kernel(MatView v, int rows, int rows_pad,
-                                                           int k0, int kn, int nkb,
-                                                           const int* __restrict__ e,
-                                                           uint16_t* __restrict__ out) {
+// Eight consecutive k of one row -> eight 16-byte chunks, one per plane.
+template <int TR>
+__device__ __forceinline__ void store_chunk(const double (&x)[8], int er, uint16_t* dst) {
+  uint32_t w[DS][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a[DS], b[DS];
+    digits_of(x[2 * j], er, a);
+    digits_of(x[2 * j + 1], er, b);
+#pragma unroll
+    for (int s = 0; s < DS; ++s) w[s][j] = pack_bf16(a[s], b[s]);
+  }
+#pragma unroll
+  for (int s = 0; s < DS; ++s)
+    *reinterpret_cast<uint4*>(dst + (size_t)s * (TR * DKB)) =
+        make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+}
+
+// Slicing of an operand whose k are adjacent in memory: `lpr` lanes (a power
+// of two) take one row, find its exponent and write its digit planes in one
+// launch; the second read of the row comes from L1/L2.  Bound by HBM (8 bytes
+// read, 16 written per element).  Tile images [rt][kb][s] of TR x 32, zero
+// beyond rows and kn.
+template <int TR>
+__global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, int rows, int rows_pad, int k0,
+                                                         int kn, int nkb, int lpr,
+                                                         int* __restrict__ e,
+                                                         uint16_t* __restrict__ out) {
   const int nch = nkb * (DKB / 8);
-  const long long total = (long long)rows_pad * nch;
+  const int lane = threadIdx.x & 31, sub = lane & (lpr - 1), per = 32 / lpr;
+  const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+       g * per < rows_pad; g += nwarp) {
+    const long long r = g * per + lane / lpr;
+    const bool live = r < rows;
+    const double* p = live ? v.p + view_row(v, r) + k0 : nullptr;
+    int em = 0;
+    if (live)
+      for (int k = sub; k < kn; k += lpr) em = max(em, biased_exponent(p[k]));
+    for (int o = lpr >> 1; o > 0; o >>= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
+    if (r >= rows_pad) continue;
+    if (sub == 0) e[r] = em;
+    const int er = row_scale(em);
+    const int rt = (int)(r / TR), rr = (int)(r % TR);
+    uint16_t* row = out + (size_t)rt * nkb * DS * (TR * DKB);
+    const bool vec = (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+    for (int kc = sub; kc < nch; kc += lpr) {
+      double x[8];
+      const int k = kc * 8;
+      if (live && vec && k + 8 <= kn) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double2 t = *reinterpret_cast<const double2*>(p + k + 2 * j);
+          x[2 * j] = t.x;
+          x[2 * j + 1] = t.y;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = live && k + j < kn ? p[k + j] : 0.0;
+      }
+      store_chunk<TR>(x, er,
+                      row + (size_t)(kc >> 2) * DS * (TR * DKB) + plane_offset(rr, (kc & 3) * 8));
+    }
+  }
+}
+
+// Operands whose rows are adjacent in memory (k strided): exponents first,
+// one lane per row and eight warps over the k of a block's segment (blockIdx.y),
+// combined by a maximum in shared and global memory (e zeroed before), ...
+constexpr int kExpSeg = 256;
+__global__ void __launch_bounds__(256) col_exponent_kernel(MatView v, int rows, int k0, int kn,
+                                                           int* __restrict__ e) {
+  __shared__ int sm[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long r = blockIdx.x * 32ll + lane;
+  const int kb = blockIdx.y * kExpSeg, ke = min(kn, kb + kExpSeg);
+  int em = 0;
+  if (r < rows) {
+    const double* p = v.p + view_row(v, r) + (long long)k0 * v.ks;
+#pragma unroll 8
+    for (int k = kb + w; k < ke; k += 8) em = max(em, biased_exponent(p[(long long)k * v.ks]));
+  }
+  sm[w][lane] = em;
+  __syncthreads();
+  if (w == 0 && r < rows) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) em = max(em, sm[q][lane]);
+    atomicMax(&e[r], em);
+  }
+}
+
+// ... then the digits: one thread per (row, 16 k), consecutive threads on
+// consecutive rows; the two 16-byte chunks of a plane it writes fill one
+// 32-byte sector of the swizzled image.
+template <int TR>
+__global__ void __launch_bounds__(256) slice_kcol_kernel(MatView v, int rows, int rows_pad, int k0,
+                                                         int kn, int nkb,
+                                                         const int* __restrict__ e,
+                                                         uint16_t* __restrict__ out) {
+  const int nc2 = nkb * (DKB / 16);
+  const long long total = (long long)rows_pad * nc2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
-    long long r;
-    int kc;
-    if (ROW_FAST) {
-      r = t % rows_pad;
-      kc = (int)(t / rows_pad);
-    } else {
-      r = t / nch;
-      kc = (int)(t % nch);
-    }
-    uint32_t dg[8][DS];
-    const int er = e[r];
-    const double* p = r < rows ? v.p + view_row(v, r) + (long long)k0 * v.ks : nullptr;
+    const long long r = t % rows_pad;
+    const int kc2 = (int)(t / rows_pad);
+    const bool live = r < rows;
+    const int er = row_scale(e[r]);
+    const double* p = live ? v.p + view_row(v, r) + (long long)k0 * v.ks : nullptr;
+    const int rt = (int)(r / TR), rr = (int)(r % TR);
+    uint16_t* tile = out + ((size_t)rt * nkb + (kc2 >> 1)) * DS * (TR * DKB);
+    double x[2][8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int k = kc * 8 + j;
-      const double x = (p && k < kn) ? p[(long long)k * v.ks] : 0.0;
-      digits_of(x, er, dg[j]);
+    for (int j = 0; j < 16; ++j) {
+      const int k = kc2 * 16 + j;
+      x[j >> 3][j & 7] = live && k < kn ? p[(long long)k * v.ks] : 0.0;
     }
-    const int rt = (int)(r / TR), rr = (int)(r % TR), kb = kc >> 2;
-    uint16_t* tile = out + ((size_t)rt * nkb + kb) * DS * (TR * DKB);
-    const int off = plane_offset(rr, (kc & 3) * 8);
 #pragma unroll
-    for (int s = 0; s < DS; ++s) {
-      uint4 w;
-      w.x = dg[0][s] | (dg[1][s] << 16);
-      w.y = dg[2][s] | (dg[3][s] << 16);
-      w.z = dg[4][s] | (dg[5][s] << 16);
-      w.w = dg[6][s] | (dg[7][s] << 16);
-      *reinterpret_cast<uint4*>(tile + (size_t)s * (TR * DKB) + off) = w;
-    }
+    for (int h = 0; h < 2; ++h)
+      store_chunk<TR>(x[h], er, tile + plane_offset(rr, (kc2 & 1) * 16 + h * 8));
   }
 }
 
@@ -188,7 +259,8 @@ struct DgArgs {
   const int* ea;       // row exponents (padded)
   const int* eb;       // column exponents (padded)
   OutView C;
-  double alpha;
+  double alpha;        // 1 when alpha_exp and negate carry it
+  int alpha_exp, negate;
   int M, N, nkb, mtn, ntn;
   int col_major_order;  // units nt-major (shared column tile adjacent)
   int a_lower, k0, accumulate;
@@ -222,20 +294,68 @@ __device__ __forceinline__ int unit_kblocks(const DgArgs& a, int mt) {
   return kend <= 0 ? 0 : min(a.nkb, (kend + DKB - 1) / DKB);
 }
 
-// FP64 value of one output element from its eight level sums (lv[L]).
-__device__ __forceinline__ double combine_levels(const float* lv, int sh) {
-  long long hi = __float2int_rn(lv[0]);
+// Accumulator of one output element over the K passes of a tile: levels 0..5
+// as an exact 64-bit integer in level-5 units (2^-49 of the row and column
+// scales; |sum| <= 2^60 for K <= KCHUNK) and levels 6..7 in FP32 level-5 units.
+struct ElemSum {
+  unsigned long long hi;
+  float tail;
+};
+// Bits of 2^23 + 2^22 (FP32): adding it to an integer |x| <= 2^22 leaves x in
+// the low bits (a conversion on the FP32 pipe; F2I runs at a quarter rate or
+// less), and the constant comes off once per tile.
+constexpr uint32_t kMagicBits = 0x4B400000u;
+constexpr float kMagic = 12582912.0f;
+constexpr unsigned long long kMagicSum =
+    (unsigned long long)kMagicBits *
+    (1ull + (1ull << 7) + (1ull << 14) + (1ull << 21) + (1ull << 28) + (1ull << 35));
+
+template <bool WIDE>
+__device__ __forceinline__ void add_levels(ElemSum& a, const float (&x)[DS]) {
+  int u[6];
 #pragma unroll
-  for (int L = 1; L < 6; ++L) hi = hi * 128 + __float2int_rn(lv[L]);  // |hi| < 2^59.1
-  const float tail = fmaf(lv[7], 0.0078125f, lv[6]) * 0.0078125f;     // level-5 units
-  const long long V = hi * 8 + __float2ll_rn(tail * 8.0f);
-  double r = (double)V;  // the one rounding
-  if (V != 0) {
-    const long long b = __double_as_longlong(r);
-    const int ex = (int)((b >> 52) & 0x7FF) + sh;
-    r = (ex > 0 && ex < 2047) ? __longlong_as_double(b + ((long long)sh << 52)) : ldexp(r, sh);
+  for (int L = 0; L < 6; ++L)
+    u[L] = WIDE ? __float2int_rn(x[L]) + (int)kMagicBits : __float_as_int(x[L] + kMagic);
+  unsigned long long v = a.hi + (unsigned long long)(long long)u[5];
+  v += (unsigned long long)((long long)u[4] * (1 << 7));
+  v += (unsigned long long)((long long)u[3] * (1 << 14));
+  v += (unsigned long long)((long long)u[2] * (1 << 21));
+  v += (unsigned long long)((long long)u[1] * (1 << 28));
+  v += (unsigned long long)(uint32_t)(u[0] << 3) << 32;  // u0 2^35 modulo 2^64
+  a.hi = v;
+  a.tail = fmaf(fmaf(x[7], 0.0078125f, x[6]), 0.0078125f, a.tail);
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void add_chunk(ElemSum* sum, const float (&lv)[DS][8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    float x[DS];
+#pragma unroll
+    for (int L = 0; L < DS; ++L) x[L] = lv[L][e];
+    add_levels<WIDE>(sum[e], x);
   }
-  return r;
+}
+
+// The FP64 value 2^sh (hi + tail), hi in level-5 units, rounded once to nearest
+// even.  Integer instructions throughout: an int64 -> FP64 conversion and an
+// FP64 multiply per element on this GPU's FP64 pipe (two lanes per clock per
+// SM) held the epilogue longer than the tile's MMAs took.
+__device__ __forceinline__ double finish_sum(long long hi, float tail, int sh) {
+  const unsigned long long mag = (unsigned long long)(hi < 0 ? -hi : hi) | (1ull << 20);
+  const int n = __clzll((long long)mag) - 2;  // (hi << n), tail 2^n within 2^62
+  const long long V = (hi << n) + __float2ll_rn(tail * __int_as_float((127 + n) << 23));
+  if (V == 0) return 0.0;
+  const unsigned long long a = (unsigned long long)(V < 0 ? -V : V);
+  const int lz = __clzll((long long)a);
+  const unsigned long long m = a << lz;  // top bit set; value = m 2^(sh - n - lz)
+  const int ex = sh - n - lz + 1086;     // biased exponent of the top bit
+  if (ex <= 0 || ex >= 2046) return ldexp((double)V, sh - n);  // subnormal, or at the top end
+  unsigned long long q = m >> 11;
+  const uint32_t rem = (uint32_t)m & 0x7FFu;
+  q += (rem > 0x400u || (rem == 0x400u && (q & 1))) ? 1 : 0;  // a carry moves into the exponent
+  const unsigned long long b = q + ((unsigned long long)(ex - 1) << 52);
+  return __longlong_as_double((long long)(b | (V < 0 ? 1ull << 63 : 0ull)));
 }
 
 __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* status) {
@@ -251,7 +371,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
       mbar_init(&ctl->empty[s], 1);
     }
     mbar_init(&ctl->afull, 1);
-    mbar_init(&ctl->aempty, 4);
+    mbar_init(&ctl->aempty, EWARPS);
     mbar_init(&ctl->fin, 1);
     ctl->abort = 0;
     fence_mbar_init();
@@ -324,6 +444,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
         if (!mbar_wait(&ctl->aempty, (nuse & 1) ^ 1, abort, status)) break;
         tc_fence_after();
         for (int kb = 0; kb < nkb; ++kb) {
+          if (kb && kb % PASS_KB == 0) {  // next K pass: the epilogue takes the sums first
+            tc_commit(&ctl->afull);
+            ++nuse;
+            if (!mbar_wait(&ctl->aempty, (nuse & 1) ^ 1, abort, status)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+          }
           if (!mbar_wait(&ctl->full[st], ph, abort, status)) {
             ok = false;
             break;
@@ -335,7 +464,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
 #pragma unroll
             for (int s = 0; s < DS; ++s) {
               const uint64_t ar = ds + (uint64_t)((s * A_PLANE + kk * 32) >> 4);
-              const uint32_t acc = (kb | kk | s) ? 1u : 0u;
+              const uint32_t acc = (kb % PASS_KB) | kk | s ? 1u : 0u;
               const uint32_t d = tmem + 64u * s;
               const int nblk = DS - s;  // column planes 0 .. 7 - s
               if (nblk > 4) {
@@ -362,50 +491,71 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
     }
   } else {
     // ------------------------------------------------------------ epilogue
-    const int q = warp & 3;  // TMEM lane quarter of this warp
+    const int q = warp & 3;              // TMEM lane quarter of this warp
+    const int c0 = ((warp - 2) >> 2) * ECOLS;  // its columns of the tile
     const int arow = 32 * q + lane;
-    const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16);
+    const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)c0;
     uint32_t nuse = 0;
-    for (long long u = blockIdx.x; u < a.total; u += gridDim.x) {
+    bool ok = true;
+    for (long long u = blockIdx.x; u < a.total && ok; u += gridDim.x) {
       int mt, nt;
       unit_tile(a, u, &mt, &nt);
-      if (unit_kblocks(a, mt) == 0) continue;
-      const bool got = mbar_wait(&ctl->afull, nuse & 1, abort, status);
-      if (!__all_sync(0xffffffffu, got)) break;
-      tc_fence_after();
-      const long long m = (long long)mt * TM + arow;
-      const bool mlive = m < a.M;
-      const int em = a.ea[m];
-      double* crow = mlive ? a.C.p + (m / a.C.rdiv) * a.C.rs_hi + (m % a.C.rdiv) * a.C.rs_lo
-                           : nullptr;
-#pragma unroll 1
-      for (int c = 0; c < TN / 16; ++c) {
-        float lv[DS][16];
+      const int np = (unit_kblocks(a, mt) + PASS_KB - 1) / PASS_KB;
+      if (np == 0) continue;
+      ElemSum sum[ECOLS];
 #pragma unroll
-        for (int L = 0; L < DS; ++L) tmem_ld16(tq + 64u * L + 16u * c, lv[L]);
-        tc_wait_ld();
-#pragma unroll
-        for (int L = 0; L < DS; ++L) ld_ready<16>(lv[L]);
-        if (c == TN / 16 - 1) {  // every TMEM read of this unit is done
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&ctl->aempty);
+      for (int e = 0; e < ECOLS; ++e) sum[e] = ElemSum{0ull, 0.f};
+      for (int p = 0; p < np; ++p, ++nuse) {
+        const bool got = mbar_wait(&ctl->afull, nuse & 1, abort, status);
+        if (!__all_sync(0xffffffffu, got)) {
+          ok = false;
+          break;
         }
+        tc_fence_after();
+        // only this part holds the MMAs of the next pass up: sums into
+        // registers, then the accumulators go back
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int n = nt * TN + 16 * c + e;
-          float l8[DS];
+        for (int c = 0; c < ECOLS / 8; ++c) {
+          float lv[DS][8];
 #pragma unroll
-          for (int L = 0; L < DS; ++L) l8[L] = lv[L][e];
-          if (mlive && n < a.N) {
-            double r = combine_levels(l8, em + a.eb[n] - 52);
+          for (int L = 0; L < DS; ++L) tmem_ld8(tq + (uint32_t)(TN * L + 8 * c), lv[L]);
+          tc_wait_ld();
+#pragma unroll
+          for (int L = 0; L < DS; ++L) ld_ready<8>(lv[L]);
+          float mx = 0.f;
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+#pragma unroll
+            for (int L = 0; L < 6; ++L) mx = fmaxf(mx, fabsf(lv[L][e]));
+          if (__any_sync(0xffffffffu, mx > 4194304.f))
+            add_chunk<true>(sum + 8 * c, lv);
+          else
+            add_chunk<false>(sum + 8 * c, lv);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl->aempty);
+      }
+      if (!ok) break;
+      const long long m = (long long)mt * TM + arow;
+      if (m < a.M) {
+        const int em = row_scale(a.ea[m]) + a.alpha_exp - 49;
+        const unsigned long long off = kMagicSum * (unsigned long long)np;
+        double* dst = a.C.p + (m / a.C.rdiv) * a.C.rs_hi + (m % a.C.rdiv) * a.C.rs_lo;
+        const int n0 = nt * TN + c0;
+        const int live = min(ECOLS, a.N - n0);
+#pragma unroll
+        for (int e = 0; e < ECOLS; ++e) {
+          if (e < live) {
+            double r = finish_sum((long long)(sum[e].hi - off), sum[e].tail,
+                                  em + row_scale(a.eb[n0 + e]));
             if (a.alpha != 1.0) r *= a.alpha;
-            double* dst = crow + (long long)n * a.C.cs;
-            *dst = a.accumulate ? *dst + r : r;
+            if (a.negate) r = -r;
+            double* d = dst + (long long)(n0 + e) * a.C.cs;
+            *d = a.accumulate ? *d + r : r;
           }
         }
       }
-      ++nuse;
     }
   }
   __syncthreads();
@@ -423,23 +573,23 @@ int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 template <int TR>
 int slice_operand(corr_context* c, const MatView& v, int rows, int rows_pad, int k0, int kn,
                   int nkb, int* e, uint16_t* out) {
-  const bool krow = v.ks == 1;  // k contiguous: warp per row, k-fast chunks
   const int cap = c->sms * 16;
-  if (krow)
-    row_exponent_kernel<true><<<std::min(ceil_div((long long)rows_pad * 32, 256), cap), 256, 0,
-                                 c->stream>>>(v, rows, rows_pad, k0, kn, e);
-  else
-    row_exponent_kernel<false><<<std::min(ceil_div(rows_pad, 256), cap), 256, 0, c->stream>>>(
-        v, rows, rows_pad, k0, kn, e);
+  if (v.ks == 1) {  // k contiguous
+    int lpr = 1;
+    while (lpr < 32 && lpr < nkb * (DKB / 8)) lpr *= 2;
+    const int grid = std::min(ceil_div((long long)rows_pad * lpr, 256), cap);
+    slice_krow_kernel<TR><<<grid, 256, 0, c->stream>>>(v, rows, rows_pad, k0, kn, nkb, lpr, e,
+                                                       out);
+    CORR_CUDA(cudaGetLastError());
+    c->launches += 1;
+    return CORR_OK;
+  }
+  CORR_CUDA(cudaMemsetAsync(e, 0, (size_t)rows_pad * 4, c->stream));
+  const dim3 eg((unsigned)ceil_div(rows, 32), (unsigned)ceil_div(kn, kExpSeg));
+  col_exponent_kernel<<<eg, 256, 0, c->stream>>>(v, rows, k0, kn, e);
   CORR_CUDA(cudaGetLastError());
-  const long long work = (long long)rows_pad * nkb * (DKB / 8);
-  const int grid = std::min(ceil_div(work, 256), cap);
-  if (krow)
-    slice_digits_kernel<TR, false><<<grid, 256, 0, c->stream>>>(v, rows, rows_pad, k0, kn, nkb,
-                                                                  e, out);
-  else
-    slice_digits_kernel<TR, true><<<grid, 256, 0, c->stream>>>(v, rows, rows_pad, k0, kn, nkb, e,
-                                                                 out);
+  const int grid = std::min(ceil_div((long long)rows_pad * nkb * (DKB / 16), 256), cap);
+  slice_kcol_kernel<TR><<<grid, 256, 0, c->stream>>>(v, rows, rows_pad, k0, kn, nkb, e, out);
   CORR_CUDA(cudaGetLastError());
   c->launches += 2;
   return CORR_OK;
@@ -449,7 +599,7 @@ int slice_operand(corr_context* c, const MatView& v, int rows, int rows_pad, int
 
 size_t dgemm_tc_workspace(int M, int N, int K) {
   const size_t mp = (size_t)ceil_div(M, TM) * TM, np = (size_t)ceil_div(N, TN) * TN;
-  const size_t kp = (size_t)ceil_div(std::min(K, KPASS), DKB) * DKB;
+  const size_t kp = (size_t)ceil_div(std::min(K, KCHUNK), DKB) * DKB;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
   return al(mp * kp * DS * 2) + al(np * kp * DS * 2) + al(mp * 4) + al(np * 4);
 }
@@ -458,7 +608,7 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
   if (g.M <= 0 || g.N <= 0) return CORR_OK;
   const int mtn = ceil_div(g.M, TM), ntn = ceil_div(g.N, TN);
   const int mp = mtn * TM, np = ntn * TN;
-  const size_t kp = (size_t)ceil_div(std::min(std::max(g.K, 1), KPASS), DKB) * DKB;
+  const size_t kp = (size_t)ceil_div(std::min(std::max(g.K, 1), KCHUNK), DKB) * DKB;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
   uint8_t* w = static_cast<uint8_t*>(ws);
   uint16_t* Ad = reinterpret_cast<uint16_t*>(w);
@@ -474,9 +624,12 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
                                    (int)kDgSmem));
     if (c->device >= 0 && c->device < 64) attr[c->device] = true;
   }
-  const int passes = std::max(1, ceil_div(g.K, KPASS));
-  for (int p = 0; p < passes; ++p) {
-    const int k0 = p * KPASS, kn = std::min(KPASS, g.K - k0);
+  const int chunks = std::max(1, ceil_div(g.K, KCHUNK));
+  // alpha = +-2^x goes into the result's exponent and sign, exactly
+  int ax = 0;
+  const bool pow2 = std::frexp(std::fabs(g.alpha), &ax) == 0.5 && ax > -64 && ax < 64;
+  for (int p = 0; p < chunks; ++p) {
+    const int k0 = p * KCHUNK, kn = std::min(KCHUNK, g.K - k0);
     const int nkb = ceil_div(std::max(kn, 1), DKB);
     if (kn > 0) {
       CORR_TRY(slice_operand<TM>(c, g.A, g.M, mp, k0, kn, nkb, ea, Ad));
@@ -493,7 +646,9 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
     a.ea = ea;
     a.eb = eb;
     a.C = g.C;
-    a.alpha = g.alpha;
+    a.alpha = pow2 ? 1.0 : g.alpha;
+    a.alpha_exp = pow2 ? ax - 1 : 0;
+    a.negate = pow2 && g.alpha < 0.0 ? 1 : 0;
     a.M = g.M;
     a.N = g.N;
     a.nkb = nkb;
