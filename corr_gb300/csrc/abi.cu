@@ -482,9 +482,13 @@ int rimp2_energy_core(corr_context* c, Carver& w, int nocc, int nvir, int naux, 
                                 (size_t)naux * nocc * nvir * 8, cudaMemcpyHostToDevice,
                                 c->stream));
     mark(c, 1);
-    CORR_CUDA(launch_energy_fp64(d_b, d_e, sh, partials, grid, c->stream));
+    const int np = launch_energy_fp64(d_b, d_e, sh, partials, grid, c->sms, c->stream);
+    if (np < 0) {
+      set_error("FP64 energy launch failed");
+      return CORR_ERR_CUDA;
+    }
     mark(c, 2);
-    CORR_CUDA(launch_energy_reduce(partials, grid, nullptr, out_e, c->stream));
+    CORR_CUDA(launch_energy_reduce(partials, np, nullptr, out_e, c->stream));
     c->launches += 2;
     return CORR_OK;
   }

@@ -158,8 +158,12 @@ int batch_enqueue(corr_context* c, int n, const corr_rimp2_instance* in, int pre
       int g = grid;
       if ((long long)g > sh.nunits) g = (int)sh.nunits;
       double* part = unit_part + (size_t)k * grid * 2;
-      CORR_CUDA(launch_energy_fp64(x.bia, x.eps, sh, part, g, c->stream));
-      CORR_CUDA(launch_energy_reduce(part, g, nullptr, out + 4 * (size_t)order[k], c->stream));
+      const int np = launch_energy_fp64(x.bia, x.eps, sh, part, g, c->sms, c->stream);
+      if (np < 0) {
+        set_error("batched FP64 energy launch failed");
+        return CORR_ERR_CUDA;
+      }
+      CORR_CUDA(launch_energy_reduce(part, np, nullptr, out + 4 * (size_t)order[k], c->stream));
     }
     c->launches += 2LL * n;
     return CORR_OK;

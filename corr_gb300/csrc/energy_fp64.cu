@@ -11,6 +11,8 @@
 // (i,j) and all (a,b) (can_mp2.cc:82-97): the (j,i) term equals the (i,j) term
 // with a and b swapped, and the (b,a) element of a pair pairs with (a,b).
 // No (ia|jb) value ever reaches global memory.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -137,12 +139,109 @@ __global__ void __launch_bounds__(128) energy_fp64_kernel(const double* __restri
   }
 }
 
+// The same sums on 8 x 8 tiles; S warps (4 or 1) share a unit and split its Q;
+// fragments straight from global memory (every unit of the same occupied pair
+// reads the same rows: L1/L2).  For small problems: a 64 x 64 tile costs the
+// FP64 pipe (two FMAs per clock per SM) 2 * 4096 FMAs per Q however few
+// virtuals there are, and there are few units to spread over the SMs.
+// nocc=5 nvir=19 naux=76, 90 units of 8 x 8 instead of 15 of 64 x 64: 7.0 us
+// instead of 210 us (14.8 us with S = 1, a chain of 19 steps).  With more units
+// than CTAs the FP64 pipe is the bound and S = 1 saves the exchange (nocc=9
+// nvir=64 naux=31: 21.3 us against 27.9 us).
+constexpr int ST = 8;
+
+template <int S>
+__global__ void __launch_bounds__(128) energy_fp64_small_kernel(const double* __restrict__ bia,
+                                                                const double* __restrict__ eps,
+                                                                EnergyShape sh,
+                                                                double* __restrict__ partials) {
+  __shared__ double part[4][4][32];
+  __shared__ double red[4][2];
+  const int o = sh.nocc, v = sh.nvir, X = sh.naux;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int sub = warp % S;  // this warp's part of its unit's Q
+  const long long rowQ = (long long)o * v;
+  double tot_os = 0.0, tot_ss = 0.0;
+  for (long long u0 = blockIdx.x * (4ll / S); u0 < sh.nunits; u0 += gridDim.x * (4ll / S)) {
+    const long long u = u0 + warp / S;
+    if (S == 1 && u >= sh.nunits) break;
+    int i, j, A, B;
+    pair_decode((int)(u / sh.ntpairs), o, &i, &j);
+    tpair_decode((int)(u % sh.ntpairs), sh.ntiles, &A, &B);
+    const int ra = A * ST + g, rb = B * ST + g;
+    const bool la = ra < v, lb = rb < v;
+    double acc1[2] = {0.0, 0.0}, acc2[2] = {0.0, 0.0};
+#pragma unroll 4
+    for (int q0 = 4 * sub; q0 < X; q0 += 4 * S) {
+      const int q = q0 + t;
+      const bool lq = q < X;
+      const double* bi = bia + (long long)q * rowQ + (long long)i * v;
+      const double* bj = bia + (long long)q * rowQ + (long long)j * v;
+      const double a1 = lq && la ? bi[ra] : 0.0, b1 = lq && lb ? bj[rb] : 0.0;
+      const double a2 = lq && la ? bj[ra] : 0.0, b2 = lq && lb ? bi[rb] : 0.0;
+      dmma(acc1, a1, b1);
+      dmma(acc2, a2, b2);
+    }
+    double d[4] = {acc1[0], acc1[1], acc2[0], acc2[1]};
+    if (S > 1) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) part[warp][k][lane] = d[k];
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        d[k] = (part[0][k][lane] + part[1][k][lane]) + (part[2][k][lane] + part[3][k][lane]);
+    }
+    if (sub == 0 && la) {
+      double los = 0.0, lss = 0.0;
+      const double eai = eps[o + ra];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int b = B * ST + 2 * t + e;
+        if (b >= v) continue;
+        const double r = 1.0 / (((eai + eps[o + b]) - eps[i]) - eps[j]);
+        const double df = d[e] - d[2 + e];
+        los += (d[e] * d[e] + d[2 + e] * d[2 + e]) * r;
+        lss += df * df * r;
+      }
+      const double fw = (A < B ? 2.0 : 1.0) * (i < j ? 1.0 : 0.5);
+      tot_os -= fw * los;
+      tot_ss -= fw * lss;
+    }
+    if (S > 1) __syncthreads();
+  }
+  tot_os = warp_sum(tot_os);
+  tot_ss = warp_sum(tot_ss);
+  if (lane == 0) {
+    red[warp][0] = tot_os;
+    red[warp][1] = tot_ss;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2)
+    partials[2 * blockIdx.x + threadIdx.x] = (red[0][threadIdx.x] + red[1][threadIdx.x]) +
+                                             (red[2][threadIdx.x] + red[3][threadIdx.x]);
+}
+
 }  // namespace
 
-cudaError_t launch_energy_fp64(const double* bia, const double* eps, const EnergyShape& sh,
-                               double* partials, int grid, cudaStream_t s) {
+int launch_energy_fp64(const double* bia, const double* eps, const EnergyShape& sh,
+                       double* partials, int grid, int sms, cudaStream_t s) {
+  // Small tiles when they give the busiest SM at most half the FMAs and the
+  // 64 x 64 units would not fill four rounds of it.
+  const EnergyShape s8 = make_energy_shape(sh.nocc, sh.nvir, sh.naux, ST);
+  const long long w64 = (sh.nunits + sms - 1) / sms * T * T;
+  const long long w8 = (s8.nunits + sms - 1) / sms * ST * ST;
+  if (sh.nunits <= 4ll * sms && 2 * w8 <= w64) {
+    const bool split = s8.nunits <= 2ll * sms;
+    const int sgrid = (int)std::min<long long>(split ? s8.nunits : (s8.nunits + 3) / 4, 2ll * sms);
+    if (split)
+      energy_fp64_small_kernel<4><<<sgrid, 128, 0, s>>>(bia, eps, s8, partials);
+    else
+      energy_fp64_small_kernel<1><<<sgrid, 128, 0, s>>>(bia, eps, s8, partials);
+    return cudaGetLastError() == cudaSuccess ? sgrid : -1;
+  }
   energy_fp64_kernel<<<grid, 128, 0, s>>>(bia, eps, sh, partials);
-  return cudaGetLastError();
+  return cudaGetLastError() == cudaSuccess ? grid : -1;
 }
 
 }  // namespace corr

@@ -177,6 +177,70 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ CU
   }
 }
 
+// Products with few or mostly padded 64 x 64 tiles: 16 x 16 tiles on 64
+// threads, 2 x 2 elements each, plain FP64 FMAs, bounds-checked loads.  The
+// FP64 pipe (two FMAs per clock per SM, DMMA included) bounds every tile shape
+// alike, so what counts is how many FMAs the busiest SM executes: a 64 x 64
+// tile costs 4096 per k however little of it is live.  24 x 24 x 24: 6.0 us
+// (40 us in one 64 x 64 tile); 13824 x 24 x 24: 22 us (77 us).
+constexpr int SBM = 16, SBK = 32;
+
+template <int TA, int TB>
+__global__ void __launch_bounds__(64) gemm_f64_small_kernel(GemmF64 g) {
+  __shared__ double sa[SBK][SBM + 1], sb[SBK][SBM + 1];
+  const int tid = threadIdx.x;
+  const int m0 = blockIdx.x * SBM, n0 = blockIdx.y * SBM, bz = blockIdx.z;
+  const double* A = g.A + (long long)bz * g.sa;
+  const double* B = g.B + (long long)bz * g.sb;
+  const int tm = (tid >> 3) * 2, tn = (tid & 7) * 2;
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  for (int k0 = 0; k0 < g.K; k0 += SBK) {
+#pragma unroll
+    for (int e = 0; e < SBM * SBK / 64; ++e) {
+      const int idx = tid + 64 * e;
+      // consecutive threads along the operand's contiguous dimension
+      const int ra = TA == 0 ? idx / SBK : idx % SBM, ka = TA == 0 ? idx % SBK : idx / SBM;
+      const int m = m0 + ra, k = k0 + ka;
+      sa[ka][ra] = m < g.M && k < g.K
+                       ? (TA == 0 ? A[(long long)m * g.lda + k] : A[(long long)k * g.lda + m])
+                       : 0.0;
+      const int rb = TB == 0 ? idx % SBM : idx / SBK, kb = TB == 0 ? idx / SBM : idx % SBK;
+      const int n = n0 + rb, kk = k0 + kb;
+      sb[kb][rb] = n < g.N && kk < g.K
+                       ? (TB == 0 ? B[(long long)kk * g.ldb + n] : B[(long long)n * g.ldb + kk])
+                       : 0.0;
+    }
+    __syncthreads();
+    const int ke = min(SBK, g.K - k0);
+    for (int k = 0; k < ke; ++k) {
+      const double a0 = sa[k][tm], a1 = sa[k][tm + 1], b0 = sb[k][tn], b1 = sb[k][tn + 1];
+      acc[0][0] = fma(a0, b0, acc[0][0]);
+      acc[0][1] = fma(a0, b1, acc[0][1]);
+      acc[1][0] = fma(a1, b0, acc[1][0]);
+      acc[1][1] = fma(a1, b1, acc[1][1]);
+    }
+    __syncthreads();
+  }
+  double* C = g.C + (long long)bz * g.sc;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int m = m0 + tm + i, n = n0 + tn + j;
+      if (m >= g.M || n >= g.N) continue;
+      double* c = C + (long long)m * g.ldc + n;
+      const double v = g.alpha * acc[i][j];
+      *c = g.beta == 0.0 ? v : v + g.beta * (*c);
+    }
+}
+
+// FMAs on the busiest of the GPU's SMs for tiles of t x t over K steps of kb.
+double busiest_sm(const GemmF64& g, int t, int kb) {
+  constexpr long long kSms = 152;
+  const long long tiles = (long long)((g.M + t - 1) / t) * ((g.N + t - 1) / t) * g.batch;
+  return (double)((tiles + kSms - 1) / kSms) * t * t * ((g.K + kb - 1) / kb * kb);
+}
+
 bool aligned16(const void* p, long long ld) {
   return ((uintptr_t)p % 16 == 0) && ((ld * 8) % 16 == 0);
 }
@@ -185,6 +249,18 @@ bool aligned16(const void* p, long long ld) {
 
 int gemm_f64(const GemmF64& g, int* status, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return CORR_OK;
+  // small tiles where they leave the busiest SM less than half the work (their
+  // loads are not pipelined, so a smaller margin is not worth taking)
+  const dim3 sgrid((g.M + SBM - 1) / SBM, (g.N + SBM - 1) / SBM, g.batch);
+  if (2.0 * busiest_sm(g, SBM, 1) <= busiest_sm(g, BM, BK) && sgrid.y <= 65535 &&
+      sgrid.z <= 65535) {
+    if (g.ta == 0 && g.tb == 0) gemm_f64_small_kernel<0, 0><<<sgrid, 64, 0, s>>>(g);
+    else if (g.ta == 0) gemm_f64_small_kernel<0, 1><<<sgrid, 64, 0, s>>>(g);
+    else if (g.tb == 0) gemm_f64_small_kernel<1, 0><<<sgrid, 64, 0, s>>>(g);
+    else gemm_f64_small_kernel<1, 1><<<sgrid, 64, 0, s>>>(g);
+    CORR_CUDA(cudaGetLastError());
+    return CORR_OK;
+  }
   CUtensorMap ta{}, tb{};
   // TMA needs 16-byte aligned base/leading dimension and batch strides
   bool tmaA = aligned16(g.A, g.lda) && (g.sa * 8) % 16 == 0 && g.K > 0;

@@ -132,9 +132,11 @@ cudaError_t launch_energy_tc_batch(const TcInst* dtab, int n, long long total, i
 cudaError_t launch_batch_reduce(const TcInst* dtab, int n, const double* partials,
                                 const int* out_index, double* out, cudaStream_t s);
 
-// FP64 form on the FP64 tensor path (energy_fp64.cu).
-cudaError_t launch_energy_fp64(const double* bia, const double* eps, const EnergyShape& sh,
-                               double* partials, int grid, cudaStream_t s);
+// FP64 form on the FP64 tensor path (energy_fp64.cu): {os, ss} partials of the
+// launch's CTAs (room for 2 sms of them); returns their number, or -1 on a
+// launch error.  grid: CTAs of the 64 x 64 kernel.
+int launch_energy_fp64(const double* bia, const double* eps, const EnergyShape& sh,
+                       double* partials, int grid, int sms, cudaStream_t s);
 constexpr int kF64Tile = 64;
 
 }  // namespace corr

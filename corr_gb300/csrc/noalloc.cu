@@ -161,8 +161,13 @@ extern "C" int corr_rimp2_energy_noalloc(int device, void* stream, int nocc, int
 
   CORR_CUDA(cudaMemsetAsync(hdr, 0, sizeof(Header), s));  // status and results start at zero
   if (!tc) {
-    CORR_CUDA(launch_energy_fp64(bia, eps, sh, partials, grid, s));
-    CORR_CUDA(launch_energy_reduce(partials, grid, nullptr, hdr->e, s));
+    const int np = launch_energy_fp64(bia, eps, sh, partials, grid,
+                                      std::min(ds.sms, kMaxGrid / 2), s);
+    if (np < 0) {
+      set_error("corr_rimp2_energy_noalloc: energy launch failed");
+      return CORR_ERR_CUDA;
+    }
+    CORR_CUDA(launch_energy_reduce(partials, np, nullptr, hdr->e, s));
   } else {
     const int scheme = scheme_for_precision(precision);
     const int fmt = format_for_scheme(scheme);
