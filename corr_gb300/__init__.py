@@ -142,8 +142,8 @@ class Context:
 
     def rimp2_gradient(self, bia, eps, nocc, nvir, naux, dbia=None, deps=None,
                        tensor_cores=False):
-        """(E, dE/dB, dE/deps) of the RI-MP2 energy: FP64 (DMMA panels and the
-        FP64 GEMM), or with tensor_cores the digit-GEMM form (FP64-accurate)."""
+        """(E, dE/dB, dE/deps) of the RI-MP2 energy, FP64-accurate: on the digit
+        GEMM (always with tensor_cores), or on the FP64 pipe in a strict context."""
         dbia = self._out(bia, tuple(bia.shape), dbia)
         deps = self._out(eps, tuple(eps.shape), deps)
         e = MP2Energy()
@@ -183,9 +183,9 @@ class Context:
         check(self._L.corr_selftest_wait_timeout(self._h, int(limit_ms)))
 
     def set_fp64_strict(self, strict=True):
-        """Plain-form metric calls (ri_metric_inv_sqrt, calculate_ri) on the
-        FP64 pipe only (True) or with the FP64-accurate digit GEMM (False,
-        the default)."""
+        """Plain-form calls (precision "fp64", the transforms and the metric) on
+        the FP64 pipe only (True) or with their large products on the
+        FP64-accurate digit GEMM (False, the default)."""
         check(self._L.corr_set_fp64_strict(self._h, 1 if strict else 0))
 
     def set_energy_tiles(self, tiles):

@@ -12,6 +12,7 @@
 #include "abi_internal.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "panel.h"
 
 namespace corr {
 
@@ -145,6 +146,7 @@ int finish_results(corr_context* c, int nres) {
     set_error("a device-side wait exceeded its time limit");
     return CORR_ERR_DEVICE_TIMEOUT;
   }
+  if (c->hres->status & kStatusNeedFp64) return kRetryFp64;
   for (int k = 0; k < nres; ++k)
     if (!std::isfinite(c->hres->e[k])) {
       set_error("non-finite energy (zero denominator or non-finite input)");
@@ -366,9 +368,11 @@ int corr_rimp2_energy(corr_context* c, int nocc, int nvir, int naux, const doubl
   CORR_CHECK_ARG((long long)nocc * nvir <= (1ll << 31) && nocc <= 46000,
                  "corr_rimp2_energy: nocc*nvir too large");
   CORR_CUDA(cudaSetDevice(c->device));
-  int st = rimp2_energy_device(c, nocc, nvir, naux, bia, eps, precision);
-  if (st != CORR_OK) return st;
-  CORR_TRY(finish_results(c, 4));
+  auto call = [&]() -> int {
+    CORR_TRY(rimp2_energy_device(c, nocc, nvir, naux, bia, eps, precision));
+    return finish_results(c, 4);
+  };
+  CORR_TRY(precision == CORR_PREC_FP64 ? with_fp64_retry(c, false, call) : call());
   out->e_ss = c->hres->e[0];
   out->e_os = c->hres->e[1];
   out->e_total = c->hres->e[2];
@@ -414,7 +418,15 @@ static int energy_grid(corr_context* c, const EnergyShape& sh, bool tc) {
   return grid;
 }
 
-size_t energy_scratch_bytes(corr_context* c, int nocc, int nvir, int naux, int precision) {
+bool energy_on_panels(const corr_context* c, int nocc, int nvir, int naux, int precision) {
+  const double ov = (double)nocc * nvir;
+  return precision == CORR_PREC_FP64 && c->digit_guard && !c->fp64_strict &&
+         ov * ov * naux >= 3e7 && ov < 1e9 && nocc <= 16384;
+}
+
+size_t energy_scratch_bytes(corr_context* c, int nocc, int nvir, int naux, int precision,
+                            bool panels) {
+  if (panels) return energy_panel_bytes(nocc, nvir, naux);
   const bool tc = precision != CORR_PREC_FP64;
   const int Qp = padded_naux(naux);
   const EnergyShape sh = make_energy_shape(nocc, nvir, naux, tc ? kTcTile : kF64Tile);
@@ -463,8 +475,18 @@ static int upload_with_row_stats(corr_context* c, const double* host_b, double* 
 
 int rimp2_energy_core(corr_context* c, Carver& w, int nocc, int nvir, int naux, const double* d_b,
                       const double* d_e, int precision, double* res, const double* host_b,
-                      int coarse) {
+                      int coarse, bool panels) {
   double* out_e = res ? res : c->dres->e;
+  if (panels) {
+    if (host_b)
+      CORR_CUDA(cudaMemcpyAsync(const_cast<double*>(d_b), host_b,
+                                (size_t)naux * nocc * nvir * 8, cudaMemcpyHostToDevice,
+                                c->stream));
+    mark(c, 1);
+    CORR_TRY(energy_from_panels(c, w, nocc, nvir, naux, d_b, d_e, out_e));
+    mark(c, 2);
+    return CORR_OK;
+  }
   const bool tc = precision != CORR_PREC_FP64;
   const int Qp = padded_naux(naux);
   const EnergyShape sh = make_energy_shape(nocc, nvir, naux, tc ? kTcTile : kF64Tile);
@@ -542,7 +564,8 @@ int rimp2_energy_device(corr_context* c, int nocc, int nvir, int naux, const dou
   if (!b_dev) cv.take(nb * 8);
   if (!e_dev) cv.take(ne * 8);
   const size_t head = cv.used;
-  CORR_TRY(c->ws.reserve(head + energy_scratch_bytes(c, nocc, nvir, naux, precision)));
+  const bool panels = !res && energy_on_panels(c, nocc, nvir, naux, precision);
+  CORR_TRY(c->ws.reserve(head + energy_scratch_bytes(c, nocc, nvir, naux, precision, panels)));
   Carver w{c->ws.ptr, 0};
   void* b_slot = b_dev ? nullptr : w.take(nb * 8);
   void* e_slot = e_dev ? nullptr : w.take(ne * 8);
@@ -557,7 +580,7 @@ int rimp2_energy_device(corr_context* c, int nocc, int nvir, int naux, const dou
     return CORR_ERR_CUDA;
   }
   return rimp2_energy_core(c, w, nocc, nvir, naux, d_b, d_e, precision, res,
-                           b_dev ? nullptr : bia);
+                           b_dev ? nullptr : bia, 0, panels);
 }
 
 }  // namespace corr

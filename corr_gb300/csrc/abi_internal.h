@@ -13,9 +13,14 @@ namespace corr {
 // Small result block the kernels write and one D2H copy brings back.
 struct ResultBlock {
   double e[8];
-  int status;  // bit flags raised by device code (CORR_ERR_DEVICE_TIMEOUT)
+  int status;  // bit flags raised by device code (CORR_ERR_DEVICE_TIMEOUT, kStatusNeedFp64)
   int pad;
 };
+
+// Status bit of the digit GEMM's range guard, and the internal result of a call
+// that has to be repeated on the FP64 pipe because of it.
+constexpr int kStatusNeedFp64 = 1 << 16;
+constexpr int kRetryFp64 = 1001;
 
 struct Workspace {
   void* ptr = nullptr;
@@ -48,7 +53,8 @@ struct corr_context {
   float t_prepass = 0.f, t_kernel = 0.f, t_total = 0.f;
   long long launches = 0;
   bool attrs_set = false;  // one-time kernel attributes (kept out of graph capture)
-  int fp64_strict = 0;     // 1: the plain-form metric calls use FP64 GEMMs and Jacobi only
+  int fp64_strict = 0;     // 1: the plain form uses the FP64 pipe only (corr_set_fp64_strict)
+  bool digit_guard = false;  // a plain-form call is running on the digit GEMM
   // batched driver
   int batch_order = 1;   // 0 input order, 1 cost-descending
   int batch_stages = 3;
@@ -84,6 +90,28 @@ namespace corr {
 const void* stage_in(corr_context* c, const void* p, size_t bytes, void* slot);
 int stage_out(corr_context* c, void* dst, const void* src, size_t bytes);
 int finish_results(corr_context* c, int nres);
+// Run a plain-form call with the digit GEMM's range guard on; when an operand
+// was out of its range (kRetryFp64), its workspace does not fit, or `fp64_only`
+// (an output overlaps an input, so the call could not be repeated), run it on
+// the FP64 pipe.
+template <class F>
+int with_fp64_retry(corr_context* c, bool fp64_only, F call) {
+  if (c->fp64_strict) return call();
+  if (!fp64_only) {
+    c->digit_guard = true;
+    const int st = call();
+    c->digit_guard = false;
+    if (st != kRetryFp64 && st != CORR_ERR_OOM) return st;
+  }
+  c->fp64_strict = 1;
+  const int st = call();
+  c->fp64_strict = 0;
+  return st;
+}
+inline bool overlaps(const void* p, size_t np, const void* q, size_t nq) {
+  const char *a = static_cast<const char*>(p), *b = static_cast<const char*>(q);
+  return a < b + nq && b < a + np;
+}
 // Record timing event k (0 start, 1 before the main kernel, 2 after it, 3 end).
 void mark(corr_context* c, int k);
 // Enqueue an RI-MP2 energy; results go to `res` (device, 4 doubles; NULL =
@@ -92,11 +120,18 @@ int rimp2_energy_device(corr_context* c, int nocc, int nvir, int naux, const dou
                         const double* eps, int precision, double* res = nullptr);
 // Scratch bytes of the energy stage, and the stage itself on device-resident
 // inputs, carving from `w` (already backed by reserved workspace).
-size_t energy_scratch_bytes(corr_context* c, int nocc, int nvir, int naux, int precision);
+size_t energy_scratch_bytes(corr_context* c, int nocc, int nvir, int naux, int precision,
+                            bool panels = false);
+// Whether the plain form's energy goes through FP64-accurate panels on the
+// digit GEMM (panel.cu) rather than the fused FP64 kernel: from (nocc nvir)^2
+// naux = 3e7 on, where the FP64 pipe needs 50 us at its full rate and the
+// panel route's launches about as long (nocc=23 nvir=211 naux=743: 33.2 ms a
+// call against 1.17 ms).
+bool energy_on_panels(const corr_context* c, int nocc, int nvir, int naux, int precision);
 // host_b (optional): B still in host memory; the precision forms upload it
 // into d_b in row chunks on the context's copy stream, each chunk's row
 // statistics starting as soon as it has landed; the FP64 form copies it first.
 int rimp2_energy_core(corr_context* c, Carver& w, int nocc, int nvir, int naux, const double* d_b,
                       const double* d_e, int precision, double* res,
-                      const double* host_b = nullptr, int coarse = 0);
+                      const double* host_b = nullptr, int coarse = 0, bool panels = false);
 }  // namespace corr

@@ -62,11 +62,14 @@ namespace {
 
 constexpr int DS = 8;                     // digit planes per operand
 constexpr int TM = 128;                   // output tile rows
-constexpr int TN = 64;                    // output tile columns
+constexpr int TN = kDgColTile;            // output tile columns
 constexpr int DKB = 32;                   // K per stage: 64-byte tile rows
 constexpr int KPASS = 512;                // K per pass (exact levels 0..5)
 constexpr int KCHUNK = 2048;              // K per launch (digit planes in the workspace)
 constexpr int PASS_KB = KPASS / DKB;
+// Rows per launch: the row operand's digit planes stay below about 1 GiB (at
+// least 256 row tiles, so that a narrow product still fills the SMs).
+constexpr size_t kRowPlaneBytes = (size_t)1 << 30;
 constexpr int A_PLANE = TM * DKB * 2;     // 8 KB
 constexpr int B_PLANE = TN * DKB * 2;     // 4 KB
 constexpr int A_BYTES = DS * A_PLANE;     // 64 KB
@@ -94,6 +97,15 @@ __device__ __forceinline__ long long view_row(const MatView& v, long long r) {
 __device__ __forceinline__ int row_scale(int em) { return em > 0 ? em - 1022 : 0; }
 __device__ __forceinline__ int biased_exponent(double x) {
   return (__double2hiint(x) >> 20) & 0x7FF;
+}
+// Nonzero exactly when x is not +-0.
+__device__ __forceinline__ uint32_t nonzero_bits(double x) {
+  return ((uint32_t)__double2hiint(x) << 1) | (uint32_t)__double2loint(x);
+}
+// Rows the splitting cannot represent: not finite, or so small that the digits
+// would lose subnormal elements.
+__device__ __forceinline__ bool row_out_of_range(int em, uint32_t nz) {
+  return em == 0x7FF || (em < 64 && nz != 0);
 }
 
 // The eight digits of x / 2^er as FP32 integers, most significant first.
@@ -154,10 +166,12 @@ __device__ __forceinline__ void store_chunk(const double (&x)[8], int er, uint16
 // read, 16 written per element).  Tile images [rt][kb][s] of TR x 32, zero
 // beyond rows and kn.
 template <int TR>
-__global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, int rows, int rows_pad, int k0,
+__global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, long long r0, int rows,
+                                                         int rows_pad, int k0,
                                                          int kn, int nkb, int lpr,
                                                          int* __restrict__ e,
-                                                         uint16_t* __restrict__ out) {
+                                                         uint16_t* __restrict__ out,
+                                                         int* __restrict__ status) {
   const int nch = nkb * (DKB / 8);
   const int lane = threadIdx.x & 31, sub = lane & (lpr - 1), per = 32 / lpr;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -165,13 +179,24 @@ __global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, int rows, in
        g * per < rows_pad; g += nwarp) {
     const long long r = g * per + lane / lpr;
     const bool live = r < rows;
-    const double* p = live ? v.p + view_row(v, r) + k0 : nullptr;
+    const double* p = live ? v.p + view_row(v, r0 + r) + k0 : nullptr;
     int em = 0;
+    uint32_t nz = 0;
     if (live)
-      for (int k = sub; k < kn; k += lpr) em = max(em, biased_exponent(p[k]));
-    for (int o = lpr >> 1; o > 0; o >>= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
+      for (int k = sub; k < kn; k += lpr) {
+        const double x = p[k];
+        em = max(em, biased_exponent(x));
+        nz |= nonzero_bits(x);
+      }
+    for (int o = lpr >> 1; o > 0; o >>= 1) {
+      em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
+      nz |= __shfl_xor_sync(0xffffffffu, nz, o);
+    }
     if (r >= rows_pad) continue;
-    if (sub == 0) e[r] = em;
+    if (sub == 0) {
+      e[r] = em;
+      if (status && row_out_of_range(em, nz)) atomicOr(status, kStatusNeedFp64);
+    }
     const int er = row_scale(em);
     const int rt = (int)(r / TR), rr = (int)(r % TR);
     uint16_t* row = out + (size_t)rt * nkb * DS * (TR * DKB);
@@ -200,24 +225,38 @@ __global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, int rows, in
 // one lane per row and eight warps over the k of a block's segment (blockIdx.y),
 // combined by a maximum in shared and global memory (e zeroed before), ...
 constexpr int kExpSeg = 256;
-__global__ void __launch_bounds__(256) col_exponent_kernel(MatView v, int rows, int k0, int kn,
-                                                           int* __restrict__ e) {
+__global__ void __launch_bounds__(256) col_exponent_kernel(MatView v, long long r0, int rows,
+                                                           int k0, int kn,
+                                                           int* __restrict__ e,
+                                                           int* __restrict__ status) {
   __shared__ int sm[8][32];
+  __shared__ uint32_t snz[8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long r = blockIdx.x * 32ll + lane;
   const int kb = blockIdx.y * kExpSeg, ke = min(kn, kb + kExpSeg);
   int em = 0;
+  uint32_t nz = 0;
   if (r < rows) {
-    const double* p = v.p + view_row(v, r) + (long long)k0 * v.ks;
+    const double* p = v.p + view_row(v, r0 + r) + (long long)k0 * v.ks;
 #pragma unroll 8
-    for (int k = kb + w; k < ke; k += 8) em = max(em, biased_exponent(p[(long long)k * v.ks]));
+    for (int k = kb + w; k < ke; k += 8) {
+      const double x = p[(long long)k * v.ks];
+      em = max(em, biased_exponent(x));
+      nz |= nonzero_bits(x);
+    }
   }
   sm[w][lane] = em;
+  snz[w][lane] = nz;
   __syncthreads();
   if (w == 0 && r < rows) {
 #pragma unroll
-    for (int q = 1; q < 8; ++q) em = max(em, sm[q][lane]);
+    for (int q = 1; q < 8; ++q) {
+      em = max(em, sm[q][lane]);
+      nz |= snz[q][lane];
+    }
     atomicMax(&e[r], em);
+    // per segment of k: a small segment of a large row also takes the FP64 pipe
+    if (status && row_out_of_range(em, nz)) atomicOr(status, kStatusNeedFp64);
   }
 }
 
@@ -225,7 +264,8 @@ __global__ void __launch_bounds__(256) col_exponent_kernel(MatView v, int rows, 
 // consecutive rows; the two 16-byte chunks of a plane it writes fill one
 // 32-byte sector of the swizzled image.
 template <int TR>
-__global__ void __launch_bounds__(256) slice_kcol_kernel(MatView v, int rows, int rows_pad, int k0,
+__global__ void __launch_bounds__(256) slice_kcol_kernel(MatView v, long long r0, int rows,
+                                                         int rows_pad, int k0,
                                                          int kn, int nkb,
                                                          const int* __restrict__ e,
                                                          uint16_t* __restrict__ out) {
@@ -237,7 +277,7 @@ __global__ void __launch_bounds__(256) slice_kcol_kernel(MatView v, int rows, in
     const int kc2 = (int)(t / rows_pad);
     const bool live = r < rows;
     const int er = row_scale(e[r]);
-    const double* p = live ? v.p + view_row(v, r) + (long long)k0 * v.ks : nullptr;
+    const double* p = live ? v.p + view_row(v, r0 + r) + (long long)k0 * v.ks : nullptr;
     const int rt = (int)(r / TR), rr = (int)(r % TR);
     uint16_t* tile = out + ((size_t)rt * nkb + (kc2 >> 1)) * DS * (TR * DKB);
     double x[2][8];
@@ -261,7 +301,8 @@ struct DgArgs {
   OutView C;
   double alpha;        // 1 when alpha_exp and negate carry it
   int alpha_exp, negate;
-  int M, N, nkb, mtn, ntn;
+  int M, N, nkb, mtn, ntn;  // M: end of this launch's rows (m0 its first)
+  int m0;
   int col_major_order;  // units nt-major (shared column tile adjacent)
   int a_lower, k0, accumulate;
   long long total;
@@ -290,7 +331,7 @@ __device__ __forceinline__ void unit_tile(const DgArgs& a, long long u, int* mt,
 // K blocks of this pass that tile row mt needs (lower-triangular A: k <= m).
 __device__ __forceinline__ int unit_kblocks(const DgArgs& a, int mt) {
   if (!a.a_lower) return a.nkb;
-  const int kend = (mt + 1) * TM - a.k0;  // local k < kend can be nonzero
+  const int kend = a.m0 + (mt + 1) * TM - a.k0;  // local k < kend can be nonzero
   return kend <= 0 ? 0 : min(a.nkb, (kend + DKB - 1) / DKB);
 }
 
@@ -537,9 +578,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
         if (lane == 0) mbar_arrive(&ctl->aempty);
       }
       if (!ok) break;
-      const long long m = (long long)mt * TM + arow;
+      const long long m = a.m0 + (long long)mt * TM + arow;
       if (m < a.M) {
-        const int em = row_scale(a.ea[m]) + a.alpha_exp - 49;
+        const int em = row_scale(a.ea[m - a.m0]) + a.alpha_exp - 49;
         const unsigned long long off = kMagicSum * (unsigned long long)np;
         double* dst = a.C.p + (m / a.C.rdiv) * a.C.rs_hi + (m % a.C.rdiv) * a.C.rs_lo;
         const int n0 = nt * TN + c0;
@@ -569,27 +610,29 @@ constexpr size_t kDgSmem = (size_t)NSTAGE * STAGE + sizeof(DgCtl) + 1024;
 static_assert(kDgSmem <= 227 * 1024, "shared memory");
 
 int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 template <int TR>
-int slice_operand(corr_context* c, const MatView& v, int rows, int rows_pad, int k0, int kn,
+int slice_operand(corr_context* c, const MatView& v, long long r0, int rows, int rows_pad, int k0, int kn,
                   int nkb, int* e, uint16_t* out) {
   const int cap = c->sms * 16;
+  int* status = c->digit_guard ? &c->dres->status : nullptr;
   if (v.ks == 1) {  // k contiguous
     int lpr = 1;
     while (lpr < 32 && lpr < nkb * (DKB / 8)) lpr *= 2;
     const int grid = std::min(ceil_div((long long)rows_pad * lpr, 256), cap);
-    slice_krow_kernel<TR><<<grid, 256, 0, c->stream>>>(v, rows, rows_pad, k0, kn, nkb, lpr, e,
-                                                       out);
+    slice_krow_kernel<TR><<<grid, 256, 0, c->stream>>>(v, r0, rows, rows_pad, k0, kn, nkb, lpr, e,
+                                                       out, status);
     CORR_CUDA(cudaGetLastError());
     c->launches += 1;
     return CORR_OK;
   }
   CORR_CUDA(cudaMemsetAsync(e, 0, (size_t)rows_pad * 4, c->stream));
   const dim3 eg((unsigned)ceil_div(rows, 32), (unsigned)ceil_div(kn, kExpSeg));
-  col_exponent_kernel<<<eg, 256, 0, c->stream>>>(v, rows, k0, kn, e);
+  col_exponent_kernel<<<eg, 256, 0, c->stream>>>(v, r0, rows, k0, kn, e, status);
   CORR_CUDA(cudaGetLastError());
   const int grid = std::min(ceil_div((long long)rows_pad * nkb * (DKB / 16), 256), cap);
-  slice_kcol_kernel<TR><<<grid, 256, 0, c->stream>>>(v, rows, rows_pad, k0, kn, nkb, e, out);
+  slice_kcol_kernel<TR><<<grid, 256, 0, c->stream>>>(v, r0, rows, rows_pad, k0, kn, nkb, e, out);
   CORR_CUDA(cudaGetLastError());
   c->launches += 2;
   return CORR_OK;
@@ -597,27 +640,56 @@ int slice_operand(corr_context* c, const MatView& v, int rows, int rows_pad, int
 
 }  // namespace
 
+// Rows of a launch for K (padded) of kp: a multiple of TM.
+static int row_chunk(int M, size_t kp) {
+  const size_t fit = kRowPlaneBytes / (kp * DS * 2) / TM * TM;
+  return (int)std::min<size_t>((size_t)ceil_div(M, TM) * TM, std::max<size_t>(fit, 256 * TM));
+}
+
 size_t dgemm_tc_workspace(int M, int N, int K) {
-  const size_t mp = (size_t)ceil_div(M, TM) * TM, np = (size_t)ceil_div(N, TN) * TN;
-  const size_t kp = (size_t)ceil_div(std::min(K, KCHUNK), DKB) * DKB;
-  auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-  return al(mp * kp * DS * 2) + al(np * kp * DS * 2) + al(mp * 4) + al(np * 4);
+  const size_t np = (size_t)ceil_div(N, TN) * TN;
+  const size_t kp = (size_t)ceil_div(std::min(std::max(K, 1), KCHUNK), DKB) * DKB;
+  const size_t mp = row_chunk(M, kp);
+  return align256(mp * kp * DS * 2) + align256(np * kp * DS * 2) + align256(mp * 4) +
+         align256(np * 4);
+}
+
+size_t dgemm_tc_columns_bytes(int rows, int K) {
+  const size_t np = (size_t)ceil_div(rows, TN) * TN;
+  const size_t kp = (size_t)ceil_div(std::max(K, 1), DKB) * DKB;
+  return align256(np * kp * DS * 2) + align256(np * 4 * ceil_div(std::max(K, 1), KCHUNK));
+}
+
+int dgemm_tc_slice_columns(corr_context* c, const MatView& v, int rows, int K, void* ws,
+                           DgColumns* out) {
+  const int np = ceil_div(rows, TN) * TN;
+  const size_t kp = (size_t)ceil_div(std::max(K, 1), DKB) * DKB;
+  uint16_t* planes = static_cast<uint16_t*>(ws);
+  int* e = reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + align256(np * kp * DS * 2));
+  for (int k0 = 0, p = 0; k0 < K; k0 += KCHUNK, ++p) {
+    const int kn = std::min(KCHUNK, K - k0);
+    CORR_TRY(slice_operand<TN>(c, v, 0, rows, np, k0, kn, ceil_div(kn, DKB), e + (size_t)p * np,
+                               planes + (size_t)p * KCHUNK * np * DS));
+  }
+  out->planes = planes;
+  out->e = e;
+  out->rows_pad = np;
+  return CORR_OK;
 }
 
 int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
   if (g.M <= 0 || g.N <= 0) return CORR_OK;
-  const int mtn = ceil_div(g.M, TM), ntn = ceil_div(g.N, TN);
-  const int mp = mtn * TM, np = ntn * TN;
+  const int ntn = ceil_div(g.N, TN), np = ntn * TN;
   const size_t kp = (size_t)ceil_div(std::min(std::max(g.K, 1), KCHUNK), DKB) * DKB;
-  auto al = [](size_t b) { return (b + 255) / 256 * 256; };
+  const int mp = row_chunk(g.M, kp);
   uint8_t* w = static_cast<uint8_t*>(ws);
   uint16_t* Ad = reinterpret_cast<uint16_t*>(w);
-  w += al((size_t)mp * kp * DS * 2);
-  uint16_t* Bd = reinterpret_cast<uint16_t*>(w);
-  w += al((size_t)np * kp * DS * 2);
+  w += align256((size_t)mp * kp * DS * 2);
   int* ea = reinterpret_cast<int*>(w);
-  w += al((size_t)mp * 4);
-  int* eb = reinterpret_cast<int*>(w);
+  w += align256((size_t)mp * 4);
+  uint16_t* Bw = reinterpret_cast<uint16_t*>(w);
+  if (!g.pre) w += align256((size_t)np * kp * DS * 2);
+  int* ebw = reinterpret_cast<int*>(w);
   static bool attr[64] = {};
   if (c->device < 0 || c->device >= 64 || !attr[c->device]) {
     CORR_CUDA(cudaFuncSetAttribute(dgemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -631,39 +703,51 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
   for (int p = 0; p < chunks; ++p) {
     const int k0 = p * KCHUNK, kn = std::min(KCHUNK, g.K - k0);
     const int nkb = ceil_div(std::max(kn, 1), DKB);
-    if (kn > 0) {
-      CORR_TRY(slice_operand<TM>(c, g.A, g.M, mp, k0, kn, nkb, ea, Ad));
-      CORR_TRY(slice_operand<TN>(c, g.B, g.N, np, k0, kn, nkb, eb, Bd));
-    } else {  // K == 0: zero digits give C = 0 (or C unchanged when accumulating)
-      CORR_CUDA(cudaMemsetAsync(Ad, 0, (size_t)mp * kp * DS * 2, c->stream));
-      CORR_CUDA(cudaMemsetAsync(Bd, 0, (size_t)np * kp * DS * 2, c->stream));
-      CORR_CUDA(cudaMemsetAsync(ea, 0, (size_t)mp * 4, c->stream));
-      CORR_CUDA(cudaMemsetAsync(eb, 0, (size_t)np * 4, c->stream));
+    const uint16_t* Bd = Bw;
+    const int* eb = ebw;
+    if (kn <= 0) {  // K == 0: zero digits give C = 0 (or C unchanged when accumulating)
+      CORR_CUDA(cudaMemsetAsync(Bw, 0, (size_t)np * kp * DS * 2, c->stream));
+      CORR_CUDA(cudaMemsetAsync(ebw, 0, (size_t)np * 4, c->stream));
+    } else if (g.pre) {
+      Bd = g.pre->planes + ((size_t)p * KCHUNK * g.pre->rows_pad + (size_t)g.col0 * nkb * DKB) * DS;
+      eb = g.pre->e + (size_t)p * g.pre->rows_pad + g.col0;
+    } else {
+      CORR_TRY(slice_operand<TN>(c, g.B, 0, g.N, np, k0, kn, nkb, ebw, Bw));
     }
-    DgArgs a;
-    a.Ad = Ad;
-    a.Bd = Bd;
-    a.ea = ea;
-    a.eb = eb;
-    a.C = g.C;
-    a.alpha = pow2 ? 1.0 : g.alpha;
-    a.alpha_exp = pow2 ? ax - 1 : 0;
-    a.negate = pow2 && g.alpha < 0.0 ? 1 : 0;
-    a.M = g.M;
-    a.N = g.N;
-    a.nkb = nkb;
-    a.mtn = mtn;
-    a.ntn = ntn;
-    // keep the larger operand's tile shared by adjacent units (L2 reuse)
-    a.col_major_order = (long long)np > (long long)mp ? 1 : 0;
-    a.a_lower = g.a_lower ? 1 : 0;
-    a.k0 = k0;
-    a.accumulate = (g.accumulate || p > 0) ? 1 : 0;
-    a.total = (long long)mtn * ntn;
-    const int grid = (int)std::min<long long>(a.total, c->sms);
-    dgemm_tc_kernel<<<grid, NTHREADS, kDgSmem, c->stream>>>(a, &c->dres->status);
-    CORR_CUDA(cudaGetLastError());
-    c->launches += 1;
+    for (int m0 = 0; m0 < g.M; m0 += mp) {
+      const int rows = std::min(mp, g.M - m0), mtn = ceil_div(rows, TM);
+      if (kn > 0) {
+        CORR_TRY(slice_operand<TM>(c, g.A, m0, rows, mtn * TM, k0, kn, nkb, ea, Ad));
+      } else {
+        CORR_CUDA(cudaMemsetAsync(Ad, 0, (size_t)mp * kp * DS * 2, c->stream));
+        CORR_CUDA(cudaMemsetAsync(ea, 0, (size_t)mp * 4, c->stream));
+      }
+      DgArgs a;
+      a.Ad = Ad;
+      a.Bd = Bd;
+      a.ea = ea;
+      a.eb = eb;
+      a.C = g.C;
+      a.alpha = pow2 ? 1.0 : g.alpha;
+      a.alpha_exp = pow2 ? ax - 1 : 0;
+      a.negate = pow2 && g.alpha < 0.0 ? 1 : 0;
+      a.M = m0 + rows;
+      a.N = g.N;
+      a.m0 = m0;
+      a.nkb = nkb;
+      a.mtn = mtn;
+      a.ntn = ntn;
+      // keep the larger operand's tile shared by adjacent units (L2 reuse)
+      a.col_major_order = ntn * TN > mtn * TM ? 1 : 0;
+      a.a_lower = g.a_lower ? 1 : 0;
+      a.k0 = k0;
+      a.accumulate = (g.accumulate || p > 0) ? 1 : 0;
+      a.total = (long long)mtn * ntn;
+      const int grid = (int)std::min<long long>(a.total, c->sms);
+      dgemm_tc_kernel<<<grid, NTHREADS, kDgSmem, c->stream>>>(a, &c->dres->status);
+      CORR_CUDA(cudaGetLastError());
+      c->launches += 1;
+    }
   }
   return CORR_OK;
 }

@@ -17,6 +17,7 @@
 // of the hot path: build_FMo, the four MOtrans quarter transforms, transform_ri,
 // the RI B build and the J^-1/2 assembly.
 #include "common.cuh"
+#include "dgemm_tc.h"
 #include "gemm_fp64.h"
 
 namespace corr {
@@ -299,6 +300,28 @@ int gemm_f64(const GemmF64& g, int* status, cudaStream_t s) {
     return CORR_ERR_CUDA;
   }
   return CORR_OK;
+}
+
+size_t gemm_plain_workspace(const corr_context* c, long long M, long long N, long long K) {
+  return digits_pay(c, M, N, K) ? dgemm_tc_workspace((int)M, (int)N, (int)K) : 0;
+}
+
+int gemm_plain(corr_context* c, const GemmF64& g, void* ws) {
+  if (!digits_pay(c, g.M, g.N, g.K) || g.batch != 1 || g.beta != 0.0) {
+    c->launches += 1;
+    return gemm_f64(g, &c->dres->status, c->stream);
+  }
+  DgemmTc d;
+  d.A = g.ta ? mat_view(g.A, 1, g.lda) : mat_view(g.A, g.lda, 1);
+  d.B = g.tb ? mat_view(g.B, g.ldb, 1) : mat_view(g.B, 1, g.ldb);
+  d.C = out_view(g.C, g.ldc, 1);
+  d.M = g.M;
+  d.N = g.N;
+  d.K = g.K;
+  d.alpha = g.alpha;
+  d.accumulate = false;
+  d.a_lower = false;
+  return dgemm_tc(c, d, ws);
 }
 
 }  // namespace corr

@@ -23,6 +23,22 @@ struct GemmF64 {
 // Enqueue C = alpha op(A) op(B) + beta C on stream s.
 int gemm_f64(const GemmF64& g, int* status, cudaStream_t s);
 
+// The plain form's product C = alpha op(A) op(B) (one matrix, beta = 0): on the
+// digit GEMM of dgemm_tc.cu where that is faster and the context does not ask
+// for the FP64 pipe (corr_set_fp64_strict), else gemm_f64.  ws:
+// gemm_plain_workspace bytes.  Values out of the digit GEMM's range raise
+// kStatusNeedFp64.
+size_t gemm_plain_workspace(const corr_context* c, long long M, long long N, long long K);
+int gemm_plain(corr_context* c, const GemmF64& g, void* ws);
+// The rule: from about 1e7 multiply-adds on, where the FP64 pipe takes 17 us at
+// its full rate of 5.9e5 per us, the slicing and one tile of the digit GEMM
+// (about 25 us in all, three launches) are the shorter way; 13824 x 24 x 24 is
+// 22 us against 30 us, 256^3 47 us against 47 us, 300 x 300 x 300 and larger
+// the digit GEMM's.
+inline bool digits_pay(const corr_context* c, long long M, long long N, long long K) {
+  return !c->fp64_strict && (double)M * N * K >= 2e7 && M <= 0x7fffff00LL && N <= 0x7fffff00LL;
+}
+
 inline GemmF64 gemm_args(const double* A, const double* B, double* C, int M, int N, int K,
                          long long lda, long long ldb, long long ldc, int ta, int tb) {
   GemmF64 g;

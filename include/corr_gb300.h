@@ -45,7 +45,11 @@ enum corr_status {
 
 /* Arithmetic of the RI-MP2 contraction (ia|jb) = sum_Q B^Q_ia B^Q_jb. */
 enum corr_precision {
-  CORR_PREC_FP64 = 0,       /* FP64 end to end (FP64 mma.sync)                   */
+  CORR_PREC_FP64 = 0,       /* the plain form: FP64 accuracy end to end.  Large
+                               products run on the FP64-accurate digit GEMM
+                               (corr_dgemm_tc), everything else and the products
+                               of a strict context (corr_set_fp64_strict) on the
+                               FP64 pipe                                         */
   CORR_PREC_SPLIT_FP16 = 1, /* each row (i,a) of B scaled by a power of two and
                                split into two integer digits s0 + s1/L stored as
                                FP16 (|digit| <= 2048); the products s0.s0',
@@ -182,12 +186,18 @@ int corr_selftest_wait_timeout(corr_context* ctx, int limit_ms);
  * columns save.) */
 int corr_set_energy_tiles(corr_context* ctx, int tiles);
 
-/* FP64 arithmetic of the plain-form metric calls (no counterpart in the
- * reference).  0 (the default): corr_ri_metric_inv_sqrt and corr_calculate_ri
- * compute J^-1/2 of a certified metric by Newton-Schulz and BPQ = J^-1/2 (Q|mn)
- * on the FP64-accurate digit GEMM (corr_dgemm_tc; 5e-11 from LAPACK's J^-1/2
- * on the 20-water cluster).  1: every product on the FP64 pipe and J^-1/2 by
- * the eigendecomposition -- IEEE FP64 end to end, several times slower. */
+/* FP64 arithmetic of the plain form (no counterpart in the reference).  0 (the
+ * default): the large products of the plain-form calls (corr_rimp2_energy and
+ * corr_rimp2_energy_from_3index with CORR_PREC_FP64, corr_rimp2_gradient,
+ * corr_transform_ri, corr_build_fmo, corr_motrans, corr_ri_build_bpq,
+ * corr_ri_apply_metric, corr_calculate_ri) run on the FP64-accurate digit GEMM
+ * (corr_dgemm_tc), and J^-1/2 of a certified metric is computed by
+ * Newton-Schulz on it (5e-11 from LAPACK's on the 20-water cluster); inputs
+ * outside the digit GEMM's range (not finite, rows of subnormals) repeat the
+ * call on the FP64 pipe.  1: every product on the FP64 pipe and J^-1/2 by the
+ * eigendecomposition -- IEEE FP64 end to end, many times slower.
+ * corr_rimp2_energy_async, the batched calls and corr_rimp2_energy_noalloc run
+ * their FP64 form on the FP64 pipe in either mode. */
 int corr_set_fp64_strict(corr_context* ctx, int strict);
 
 /* Launch variant of the batched kernel: unit order (0 = input order,
@@ -204,7 +214,8 @@ int corr_rimp2_batch_autotune(corr_context* ctx, int n, const corr_rimp2_instanc
 
 /* RI-MP2 adjoint (no counterpart in the reference, which has no gradients):
  * dbia[(Q*nocc+i)*nvir+a] = dE/dB^Q_ia and deps[p] = dE/d eps_p for
- * E = E_OS + E_SS of corr_rimp2_energy, in FP64.  The (ia|jb) tiles are
+ * E = E_OS + E_SS of corr_rimp2_energy, to FP64 accuracy (on the digit GEMM, or
+ * on the FP64 pipe in a strict context).  The (ia|jb) tiles are
  * recomputed, never stored: per block of occupied orbitals a transient panel
  * G^{ij}_ab = -(4 (ia|jb) - 2 (ib|ja)) / D (at most ~1 GiB) feeds one GEMM
  * dB = 2 B G^T; dE/d eps comes from W = (2(ia|jb) - (ib|ja))(ia|jb)/D^2.
@@ -213,8 +224,9 @@ int corr_rimp2_gradient(corr_context* ctx, int nocc, int nvir, int naux, const d
                         const double* eps, double* dbia, double* deps, corr_mp2_energy* e_out);
 
 /* corr_rimp2_gradient on the tensor cores: per block of occupied orbitals the
- * panel (ia|jb) by the FP64-accurate digit GEMM (corr_dgemm_tc), G, W and E
- * in place, and dB = 2 B G^T by the digit GEMM; the same outputs to the digit
+ * panel (ia|jb), j not before the block, by the FP64-accurate digit GEMM
+ * (corr_dgemm_tc), G, W and E in place, and both products of the symmetric
+ * panel with B into dB by the digit GEMM; the same outputs to the digit
  * GEMM's accuracy (~FP64), at tensor-core speed.  nvir <= 6144.  The adjoint
  * of the precision forms (the autograd backward of a split-precision
  * forward). */
@@ -244,7 +256,7 @@ int corr_rimp2_energy_noalloc(int device, void* stream, int nocc, int nvir, int 
 
 /* Replaces build_FMo (src/POSTHF/motrans.cc:8-32, declared at
  * src/POSTHF/motrans.h:22): fmo[i*N+j] = sum_{mu,nu} mos[i*N+mu] fmat[mu*N+nu]
- * mos[j*N+nu], as two FP64 GEMMs.  The caller owns fmo (N*N). */
+ * mos[j*N+nu], as two FP64-accurate GEMMs.  The caller owns fmo (N*N). */
 int corr_build_fmo(corr_context* ctx, int nroao, const double* mos, const double* fmat,
                    double* fmo);
 
