@@ -20,6 +20,7 @@
 #include "dgemm_tc.h"
 #include "gemm_fp64.h"
 #include "kernels.h"
+#include "panel.h"
 
 namespace corr {
 
@@ -177,77 +178,6 @@ __global__ void __launch_bounds__(128) adjoint_panel_kernel(PanelArgs g) {
   }
 }
 
-// Tensor-core form, step 2: the panel P[(il, a)][(j, b)] holds M^{ij}_ab for
-// the occupied block i = i0 + il; one CTA per (il, j) replaces every element
-// by G^{ij}_ab = -(4 M_ab - 2 M_ba) / D (in place: one thread owns the pair
-// (a, b), (b, a)), accumulates W = (2 M_ab - M_ba) M_ab / D^2 into dE/d eps
-// (per-CTA sums in shared memory, then atomics) and writes the pair block's
-// energy -sum (2 M_ab - M_ba) M_ab / D to its own partial.
-__global__ void __launch_bounds__(256) grad_panel_kernel(double* __restrict__ P,
-                                                         const double* __restrict__ eps, int o,
-                                                         int v, int i0, double* __restrict__ deps,
-                                                         double* __restrict__ part) {
-  extern __shared__ double wv[];  // [v]: W summed into dE/d eps_(o+c)
-  __shared__ double red[2][8];
-  const int il = blockIdx.x / o, j = blockIdx.x % o, i = i0 + il;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int c = threadIdx.x; c < v; c += blockDim.x) wv[c] = 0.0;
-  __syncthreads();
-  const long long ld = (long long)o * v;
-  double* Pi = P + (long long)il * v * ld + (long long)j * v;  // row a at Pi + a * ld
-  const double eij = eps[i] + eps[j];
-  double wsum = 0.0, esum = 0.0;
-  for (int a = warp; a < v; a += nw) {
-    const double ea = eps[o + a];
-    double wa = 0.0;
-    for (int b = a + lane; b < v; b += 32) {
-      const double r = 1.0 / ((ea + eps[o + b]) - eij);
-      double* pab = Pi + (long long)a * ld + b;
-      double* pba = Pi + (long long)b * ld + a;
-      const double mab = *pab, mba = *pba;
-      const double tab = 2.0 * mab - mba, tba = 2.0 * mba - mab;
-      double w, e;
-      if (a == b) {
-        w = 2.0 * tab * mab * r * r;  // (a == c) and (b == c)
-        e = tab * mab * r;
-        *pab = -2.0 * tab * r;
-      } else {
-        const double wab = (tab * mab + tba * mba) * r * r;
-        w = wab;
-        e = (tab * mab + tba * mba) * r;
-        *pab = -2.0 * tab * r;
-        *pba = -2.0 * tba * r;
-        atomicAdd(&wv[b], wab);
-      }
-      wa += w;
-      wsum += (a == b) ? 0.5 * w : w;
-      esum -= e;
-    }
-    for (int off = 16; off > 0; off >>= 1) wa += __shfl_xor_sync(0xffffffffu, wa, off);
-    if (lane == 0) atomicAdd(&wv[a], wa);
-  }
-  wsum = warp_sum(wsum);
-  esum = warp_sum(esum);
-  if (lane == 0) {
-    red[0][warp] = wsum;
-    red[1][warp] = esum;
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < v; c += blockDim.x)
-    if (wv[c] != 0.0) atomicAdd(&deps[o + c], wv[c]);
-  if (threadIdx.x == 0) {
-    double ws = 0.0, es = 0.0;
-    for (int k = 0; k < nw; ++k) {
-      ws += red[0][k];
-      es += red[1][k];
-    }
-    atomicAdd(&deps[i], -ws);
-    atomicAdd(&deps[j], -ws);
-    part[2 * blockIdx.x] = es;
-    part[2 * blockIdx.x + 1] = 0.0;
-  }
-}
-
 }  // namespace
 
 size_t rimp2_gradient_workspace(int o, int v, int sms, size_t panel_budget);
@@ -303,63 +233,75 @@ size_t rimp2_gradient_workspace(int o, int v, int sms, size_t panel_budget) {
   return per_i * bi + (size_t)sms * 2 * 16 * ((o + bi - 1) / bi) + 512;
 }
 
-// The adjoint on the tensor cores: per block of bi occupied orbitals the
-// panel M[(i, a)][(j, b)] = sum_Q B^Q_ia B^Q_jb (i in the block, all j) by the
-// FP64-accurate digit GEMM (dgemm_tc.cu), G, W and E by grad_panel_kernel,
-// then dB[Q][(i, a)] = 2 sum_(j,b) B[Q][(j, b)] G[(i, a)][(j, b)] by the digit
-// GEMM.  FP64 accuracy (bounds of the digit GEMM), tensor-core speed.
-size_t rimp2_gradient_tc_workspace(int o, int v, int X, size_t panel_budget, int* bi_out) {
-  const size_t per_i = (size_t)v * o * v * 8;
-  int bi = (int)(panel_budget / per_i);
-  bi = std::max(1, std::min(bi, o));
-  if (bi_out) *bi_out = bi;
-  const int ov = o * v;
-  const size_t ws = std::max(dgemm_tc_workspace(bi * v, ov, X), dgemm_tc_workspace(X, bi * v, ov));
-  return per_i * bi + ws + (size_t)o * o * 16 + 1024;
+// The adjoint on the tensor cores (FP64-accurate digit GEMM, dgemm_tc.cu), per
+// block I of occupied orbitals and all j >= i0 (panel.cu):
+//   M[(i, a)][(j, b)] = sum_Q B^Q_ia B^Q_jb, then G, W and E in place,
+//   dB[Q][(i, a)] += 2 sum_(j,b) G[(i, a)][(j, b)] B[Q][(j, b)]   (j >= i0),
+//   dB[Q][(j, b)] += 2 sum_(i,a) G[(i, a)][(j, b)] B[Q][(i, a)]   (j beyond I),
+// the second by G^{ji}_ba = G^{ij}_ab: (ia|jb) is formed for half of the pairs.
+static size_t gradient_product_workspace(int o, int v, int X, int ni) {
+  const int R = o * v;
+  return std::max(std::max(dgemm_tc_workspace(ni * v, kDgColTile, X),
+                           dgemm_tc_workspace(X, ni * v, R)),
+                  dgemm_tc_workspace(X, R, ni * v));
+}
+
+size_t rimp2_gradient_tc_workspace(int o, int v, int X, size_t panel_budget) {
+  const PanelPlan p = panel_plan(o, v, X, panel_budget);
+  return p.panel_bytes + p.col_bytes + gradient_product_workspace(o, v, X, p.ni) +
+         (size_t)p.partials * 16 + (size_t)kReduceBlocks * 16 + 8 * 256;
 }
 
 int rimp2_gradient_tc(corr_context* c, Carver& w, int o, int v, int X, const double* bia,
                       const double* eps, double* dbia, double* deps, size_t panel_budget) {
   CORR_CHECK_ARG(v <= 6144, "corr_rimp2_gradient_tc: nvir %d above 6144", v);
-  int bi = 1;
-  rimp2_gradient_tc_workspace(o, v, X, panel_budget, &bi);
-  const int ov = o * v;
-  double* panel = static_cast<double*>(w.take((size_t)v * o * v * 8 * bi));
-  void* dws = w.take(std::max(dgemm_tc_workspace(bi * v, ov, X),
-                              dgemm_tc_workspace(X, bi * v, ov)));
-  double* part = static_cast<double*>(w.take((size_t)o * o * 16));
+  const PanelPlan p = panel_plan(o, v, X, panel_budget);
+  const int R = o * v;
+  double* panel = static_cast<double*>(w.take(p.panel_bytes));
+  void* cws = w.take(p.col_bytes);
+  void* dws = w.take(gradient_product_workspace(o, v, X, p.ni));
+  double* part = static_cast<double*>(w.take((size_t)p.partials * 16));
+  unsigned* ticket = static_cast<unsigned*>(w.take(16));
+  double* scratch = static_cast<double*>(w.take((size_t)kReduceBlocks * 16));
   CORR_CUDA(cudaMemsetAsync(deps, 0, (size_t)(o + v) * 8, c->stream));
-  for (int i0 = 0; i0 < o; i0 += bi) {
-    const int nb = std::min(bi, o - i0);
-    DgemmTc m;
-    m.A = mat_view(bia + (size_t)i0 * v, 1, ov);  // rows (i, a) of the block, over Q
-    m.B = mat_view(bia, 1, ov);                   // rows (j, b), over Q
-    m.C = out_view(panel, ov, 1);
-    m.M = nb * v;
-    m.N = ov;
-    m.K = X;
-    m.alpha = 1.0;
-    m.accumulate = false;
-    m.a_lower = false;
-    CORR_TRY(dgemm_tc(c, m, dws));
-    grad_panel_kernel<<<nb * o, 256, (size_t)v * 8, c->stream>>>(panel, eps, o, v, i0, deps,
-                                                                  part + (size_t)i0 * o * 2);
-    CORR_CUDA(cudaGetLastError());
+  DgColumns cols;
+  CORR_TRY(dgemm_tc_slice_columns(c, mat_view(bia, 1, R), R, X, cws, &cols));
+  long long np = 0;
+  for (int i0 = 0; i0 < o; i0 += p.ni) {
+    const int ni = std::min(p.ni, o - i0);
+    const long long r0 = (long long)i0 * v, r1 = (long long)(i0 + ni) * v;
+    PanelView pv;
+    CORR_TRY(panel_product(c, o, v, X, bia, cols, i0, ni, panel, dws, &pv));
+    CORR_TRY(launch_panel(c, pv, eps, deps, part + 2 * np, true));
+    np += (long long)ni * (o - i0);
     DgemmTc d;
-    d.A = mat_view(bia, ov, 1);    // rows Q, over (j, b)
-    d.B = mat_view(panel, ov, 1);  // rows (i, a) of the block, over (j, b)
-    d.C = out_view(dbia + (size_t)i0 * v, ov, 1);
+    d.A = mat_view(bia + r0, R, 1);                        // rows Q, over (j, b)
+    d.B = mat_view(panel + (r0 - pv.col0), pv.ld, 1);      // rows (i, a), over (j, b)
+    d.C = out_view(dbia + r0, R, 1);
     d.M = X;
-    d.N = nb * v;
-    d.K = ov;
+    d.N = ni * v;
+    d.K = (int)(R - r0);
     d.alpha = 2.0;
-    d.accumulate = false;
+    d.accumulate = i0 > 0;
     d.a_lower = false;
     CORR_TRY(dgemm_tc(c, d, dws));
-    c->launches += 1;
+    if (r1 < R) {
+      d.A = mat_view(bia + r0, R, 1);                      // rows Q, over (i, a)
+      d.B = mat_view(panel + (r1 - pv.col0), 1, pv.ld);    // rows (j, b), over (i, a)
+      d.C = out_view(dbia + r1, R, 1);
+      d.N = (int)(R - r1);
+      d.K = ni * v;
+      CORR_TRY(dgemm_tc(c, d, dws));
+    }
   }
-  CORR_CUDA(launch_energy_reduce(part, o * o, nullptr, c->dres->e, c->stream));
-  c->launches += 1;
+  CORR_CUDA(cudaMemsetAsync(ticket, 0, 16, c->stream));
+  const int nr = launch_unit_reduce(part, (int)np, nullptr, c->dres->e, scratch, ticket,
+                                    c->stream);
+  if (nr < 0) {
+    set_error("energy reduction launch failed");
+    return CORR_ERR_CUDA;
+  }
+  c->launches += nr;
   return CORR_OK;
 }
 
@@ -388,7 +330,7 @@ static int rimp2_gradient_call(corr_context* c, int nocc, int nvir, int naux, co
   double *db, *de;
   Carver cv{nullptr, 0};
   plan(cv, &sb, &se, &db, &de);
-  cv.take(tc ? rimp2_gradient_tc_workspace(nocc, nvir, naux, budget, nullptr)
+  cv.take(tc ? rimp2_gradient_tc_workspace(nocc, nvir, naux, budget)
              : rimp2_gradient_workspace(nocc, nvir, c->sms, budget));
   CORR_TRY(c->ws.reserve(cv.used));
   Carver w{c->ws.ptr, 0};
@@ -417,7 +359,18 @@ static int rimp2_gradient_call(corr_context* c, int nocc, int nvir, int naux, co
 extern "C" int corr_rimp2_gradient(corr_context* c, int nocc, int nvir, int naux,
                                    const double* bia, const double* eps, double* dbia,
                                    double* deps, corr_mp2_energy* e_out) {
-  return rimp2_gradient_call(c, nocc, nvir, naux, bia, eps, dbia, deps, e_out, false);
+  CORR_CHECK_ARG(c != nullptr, "corr_rimp2_gradient: null context");
+  // the digit GEMM unless the context asks for the FP64 pipe (or an output
+  // overlaps an input, or nvir is beyond that form's limit)
+  const size_t nb = (size_t)std::max(nocc, 0) * std::max(nvir, 0) * std::max(naux, 0) * 8;
+  const size_t ne = ((size_t)std::max(nocc, 0) + std::max(nvir, 0)) * 8;
+  const bool fp64_only = nvir > 6144 || nocc > 16384 || overlaps(dbia, nb, bia, nb) ||
+                         overlaps(deps, ne, eps, ne) || overlaps(dbia, nb, eps, ne) ||
+                         overlaps(deps, ne, bia, nb);
+  return with_fp64_retry(c, fp64_only, [&]() -> int {
+    return rimp2_gradient_call(c, nocc, nvir, naux, bia, eps, dbia, deps, e_out,
+                               c->digit_guard && !c->fp64_strict);
+  });
 }
 
 extern "C" int corr_rimp2_gradient_tc(corr_context* c, int nocc, int nvir, int naux,
