@@ -299,8 +299,9 @@ struct DgArgs {
   const int* ea;       // row exponents (padded)
   const int* eb;       // column exponents (padded)
   OutView C;
-  double alpha;        // 1 when alpha_exp and negate carry it
-  int alpha_exp, negate;
+  double alpha;        // applied when `scaled`; else alpha = +-2^alpha_exp, its sign bit in `sign`
+  int alpha_exp, scaled;
+  uint32_t sign;
   int M, N, nkb, mtn, ntn;  // M: end of this launch's rows (m0 its first)
   int m0;
   int col_major_order;  // units nt-major (shared column tile adjacent)
@@ -379,24 +380,38 @@ __device__ __forceinline__ void add_chunk(ElemSum* sum, const float (&lv)[DS][8]
 }
 
 // The FP64 value 2^sh (hi + tail), hi in level-5 units, rounded once to nearest
-// even.  Integer instructions throughout: an int64 -> FP64 conversion and an
-// FP64 multiply per element on this GPU's FP64 pipe (two lanes per clock per
-// SM) held the epilogue longer than the tile's MMAs took.
-__device__ __forceinline__ double finish_sum(long long hi, float tail, int sh) {
-  const unsigned long long mag = (unsigned long long)(hi < 0 ? -hi : hi) | (1ull << 20);
-  const int n = __clzll((long long)mag) - 2;  // (hi << n), tail 2^n within 2^62
-  const long long V = (hi << n) + __float2ll_rn(tail * __int_as_float((127 + n) << 23));
-  if (V == 0) return 0.0;
+// even.  32-bit integer and FP32 instructions throughout: this GPU's FP64 pipe
+// takes two lanes per clock per SM, so one FP64 instruction per element --
+// a 64-bit conversion, a multiply by alpha = 1, a negation -- is 2 us of a tile.
+// tail goes in at 2^-11 of a level-5 unit (2^-60 of the scales), fewer bits
+// when hi is that large.  No branches, so that eight elements overlap; *odd is
+// set for a value at the ends of the exponent range (finish_slow).
+__device__ __forceinline__ unsigned long long finish_sum(long long hi, float tail, int sh,
+                                                         uint32_t sign, bool* odd) {
+  const int hh = (int)(hi >> 32);
+  const int n = min(11, __clz(hh ^ (hh >> 31)) - 2);  // hi << n within 2^62; |hi| < 2^61
+  const long long V = (hi << n) + (__float2int_rn(tail * 2048.f) >> (11 - n));  // |tail| < 2^20
   const unsigned long long a = (unsigned long long)(V < 0 ? -V : V);
-  const int lz = __clzll((long long)a);
+  const int lz = __clzll((long long)a) & 63;
   const unsigned long long m = a << lz;  // top bit set; value = m 2^(sh - n - lz)
   const int ex = sh - n - lz + 1086;     // biased exponent of the top bit
-  if (ex <= 0 || ex >= 2046) return ldexp((double)V, sh - n);  // subnormal, or at the top end
-  unsigned long long q = m >> 11;
   const uint32_t rem = (uint32_t)m & 0x7FFu;
-  q += (rem > 0x400u || (rem == 0x400u && (q & 1))) ? 1 : 0;  // a carry moves into the exponent
-  const unsigned long long b = q + ((unsigned long long)(ex - 1) << 52);
-  return __longlong_as_double((long long)(b | (V < 0 ? 1ull << 63 : 0ull)));
+  unsigned long long b = m >> 11;
+  b += (rem + (uint32_t)(b & 1)) > 0x400u ? 1 : 0;  // to nearest even; a carry moves up
+  b += (unsigned long long)(uint32_t)(ex - 1) << 52;
+  const bool zero = a == 0;
+  *odd = !zero && (ex <= 0 || ex >= 2046);
+  b |= (unsigned long long)(sign ^ (V < 0 ? 0x80000000u : 0u)) << 32;
+  return zero ? 0ull : b;
+}
+
+// The same at the ends of the exponent range: subnormal, or near the largest.
+__device__ __noinline__ double finish_slow(long long hi, float tail, int sh, uint32_t sign) {
+  const int hh = (int)(hi >> 32);
+  const int n = min(11, __clz(hh ^ (hh >> 31)) - 2);
+  const long long V = (hi << n) + (__float2int_rn(tail * 2048.f) >> (11 - n));
+  const double r = ldexp((double)V, sh - n);
+  return sign ? -r : r;
 }
 
 __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* status) {
@@ -578,24 +593,58 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
         if (lane == 0) mbar_arrive(&ctl->aempty);
       }
       if (!ok) break;
+      // Normalise and store, eight columns per step: a rolled loop that moves
+      // the remaining sums down the register array (unrolled over 32 columns the
+      // code ran at the rate of its instruction fetches).
       const long long m = a.m0 + (long long)mt * TM + arow;
-      if (m < a.M) {
-        const int em = row_scale(a.ea[m - a.m0]) + a.alpha_exp - 49;
-        const unsigned long long off = kMagicSum * (unsigned long long)np;
-        double* dst = a.C.p + (m / a.C.rdiv) * a.C.rs_hi + (m % a.C.rdiv) * a.C.rs_lo;
-        const int n0 = nt * TN + c0;
-        const int live = min(ECOLS, a.N - n0);
+      const bool mlive = m < a.M;
+      const int n0 = nt * TN + c0;
+      const int em = (mlive ? row_scale(a.ea[m - a.m0]) : 0) + a.alpha_exp - 49;
+      const int en = row_scale(a.eb[n0 + lane]);
+      const unsigned long long off = kMagicSum * (unsigned long long)np;
+      double* dst = a.C.p + (m / a.C.rdiv) * a.C.rs_hi + (m % a.C.rdiv) * a.C.rs_lo +
+                    (long long)n0 * a.C.cs;
+      const bool vec = a.C.cs == 1 && !a.accumulate && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+#pragma unroll 1
+      for (int c = 0; c < ECOLS; c += 8) {
+        double r[8];
+        uint32_t odd = 0;
 #pragma unroll
-        for (int e = 0; e < ECOLS; ++e) {
-          if (e < live) {
-            double r = finish_sum((long long)(sum[e].hi - off), sum[e].tail,
-                                  em + row_scale(a.eb[n0 + e]));
-            if (a.alpha != 1.0) r *= a.alpha;
-            if (a.negate) r = -r;
-            double* d = dst + (long long)(n0 + e) * a.C.cs;
-            *d = a.accumulate ? *d + r : r;
+        for (int e = 0; e < 8; ++e) {
+          bool x;
+          r[e] = __longlong_as_double((long long)finish_sum(
+              (long long)(sum[e].hi - off), sum[e].tail,
+              em + __shfl_sync(0xffffffffu, en, c + e), a.sign, &x));
+          odd |= x ? 1u << e : 0u;
+        }
+        if (__any_sync(0xffffffffu, odd != 0)) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int sh = em + __shfl_sync(0xffffffffu, en, c + e);
+            if (odd >> e & 1)
+              r[e] = finish_slow((long long)(sum[e].hi - off), sum[e].tail, sh, a.sign);
           }
         }
+        if (a.scaled) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) r[e] *= a.alpha;
+        }
+        const int live = mlive ? min(8, a.N - n0 - c) : 0;
+        double* d = dst + (long long)c * a.C.cs;
+        if (vec && live == 8) {
+#pragma unroll
+          for (int e = 0; e < 8; e += 2)
+            *reinterpret_cast<double2*>(d + e) = make_double2(r[e], r[e + 1]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (e < live) {
+              double* x = d + (long long)e * a.C.cs;
+              *x = a.accumulate ? *x + r[e] : r[e];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e + 8 < ECOLS; ++e) sum[e] = sum[e + 8];
       }
     }
   }
@@ -728,9 +777,10 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
       a.ea = ea;
       a.eb = eb;
       a.C = g.C;
-      a.alpha = pow2 ? 1.0 : g.alpha;
+      a.alpha = g.alpha;
+      a.scaled = pow2 ? 0 : 1;
       a.alpha_exp = pow2 ? ax - 1 : 0;
-      a.negate = pow2 && g.alpha < 0.0 ? 1 : 0;
+      a.sign = pow2 && g.alpha < 0.0 ? 0x80000000u : 0u;
       a.M = m0 + rows;
       a.N = g.N;
       a.m0 = m0;
