@@ -306,6 +306,10 @@ struct DgArgs {
   int m0;
   int col_major_order;  // units nt-major (shared column tile adjacent)
   int a_lower, k0, accumulate;
+  int nsplit, kper;  // parts of a tile's K blocks (kper each): units are (tile, part)
+  unsigned long long* part_hi;  // nsplit > 1: [unit][warp][column][lane] sums of the parts,
+  float* part_tail;             // and per (tile, warp) the parts that have arrived
+  unsigned* ticket;
   long long total;
 };
 
@@ -319,7 +323,9 @@ struct DgCtl {
   int abort;
 };
 
+// Unit u: its tile, and the part of its K blocks.
 __device__ __forceinline__ void unit_tile(const DgArgs& a, long long u, int* mt, int* nt) {
+  if (a.nsplit > 1) u /= a.nsplit;
   if (a.col_major_order) {
     *nt = (int)(u / a.mtn);
     *mt = (int)(u % a.mtn);
@@ -334,6 +340,15 @@ __device__ __forceinline__ int unit_kblocks(const DgArgs& a, int mt) {
   if (!a.a_lower) return a.nkb;
   const int kend = a.m0 + (mt + 1) * TM - a.k0;  // local k < kend can be nonzero
   return kend <= 0 ? 0 : min(a.nkb, (kend + DKB - 1) / DKB);
+}
+
+// K blocks [*kb0, *kb1) of unit u (empty past a triangular tile's last block).
+__device__ __forceinline__ void unit_range(const DgArgs& a, long long u, int mt, int* kb0,
+                                           int* kb1) {
+  const int n = unit_kblocks(a, mt);
+  const int part = a.nsplit > 1 ? (int)(u % a.nsplit) : 0;
+  *kb0 = part * a.kper;
+  *kb1 = min(n, *kb0 + a.kper);
 }
 
 // Accumulator of one output element over the K passes of a tile: levels 0..5
@@ -450,8 +465,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
     for (long long u = blockIdx.x; u < a.total && ok; u += gridDim.x) {
       int mt, nt;
       unit_tile(a, u, &mt, &nt);
-      const int nkb = unit_kblocks(a, mt);
-      for (int kb = 0; kb < nkb; ++kb) {
+      int kb0, kb1;
+      unit_range(a, u, mt, &kb0, &kb1);
+      for (int kb = kb0; kb < kb1; ++kb) {
         bool got = true;
         if (lane == 0) got = mbar_wait(&ctl->empty[st], ph ^ 1, abort, status);
         if (!__shfl_sync(0xffffffffu, got ? 1 : 0, 0)) {
@@ -495,11 +511,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
       for (long long u = blockIdx.x; u < a.total && ok; u += gridDim.x) {
         int mt, nt;
         unit_tile(a, u, &mt, &nt);
-        const int nkb = unit_kblocks(a, mt);
-        if (nkb == 0) continue;
+        int kb0, kb1;
+        unit_range(a, u, mt, &kb0, &kb1);
+        if (kb1 <= kb0) continue;
         if (!mbar_wait(&ctl->aempty, (nuse & 1) ^ 1, abort, status)) break;
         tc_fence_after();
-        for (int kb = 0; kb < nkb; ++kb) {
+        for (int kb = 0; kb < kb1 - kb0; ++kb) {
           if (kb && kb % PASS_KB == 0) {  // next K pass: the epilogue takes the sums first
             tc_commit(&ctl->afull);
             ++nuse;
@@ -556,8 +573,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
     for (long long u = blockIdx.x; u < a.total && ok; u += gridDim.x) {
       int mt, nt;
       unit_tile(a, u, &mt, &nt);
-      const int np = (unit_kblocks(a, mt) + PASS_KB - 1) / PASS_KB;
-      if (np == 0) continue;
+      int kb0, kb1;
+      unit_range(a, u, mt, &kb0, &kb1);
+      if (kb1 <= kb0) continue;
+      const int np = (kb1 - kb0 + PASS_KB - 1) / PASS_KB;
       ElemSum sum[ECOLS];
 #pragma unroll
       for (int e = 0; e < ECOLS; ++e) sum[e] = ElemSum{0ull, 0.f};
@@ -593,6 +612,40 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
         if (lane == 0) mbar_arrive(&ctl->aempty);
       }
       if (!ok) break;
+      // the magic constants of the conversions come off once per tile
+      const unsigned long long off = kMagicSum * (unsigned long long)np;
+#pragma unroll
+      for (int e = 0; e < ECOLS; ++e) sum[e].hi -= off;
+      if (a.nsplit > 1) {
+        // A part of the tile's K: the warp leaves its sums in L2, and the warp
+        // that arrives last adds the parts up (integers exactly, the FP32 tails
+        // in part order) and stores the result.  No warp waits for another.
+        const size_t slot = ((size_t)u * EWARPS + (warp - 2)) * ECOLS * 32 + lane;
+#pragma unroll
+        for (int e = 0; e < ECOLS; ++e) {
+          __stcg(&a.part_hi[slot + 32 * e], sum[e].hi);
+          __stcg(&a.part_tail[slot + 32 * e], sum[e].tail);
+        }
+        __threadfence();
+        __syncwarp();
+        const int parts = (unit_kblocks(a, mt) + a.kper - 1) / a.kper;
+        unsigned t = 0;
+        if (lane == 0) t = atomicAdd(&a.ticket[u / a.nsplit * EWARPS + (warp - 2)], 1u);
+        if (__shfl_sync(0xffffffffu, t, 0) != (unsigned)parts - 1) continue;
+        __threadfence();
+        const size_t first =
+            ((size_t)(u / a.nsplit * a.nsplit) * EWARPS + (warp - 2)) * ECOLS * 32 + lane;
+#pragma unroll
+        for (int e = 0; e < ECOLS; ++e) sum[e] = ElemSum{0ull, 0.f};
+        for (int p = 0; p < parts; ++p) {
+          const size_t at = first + (size_t)p * EWARPS * ECOLS * 32;
+#pragma unroll
+          for (int e = 0; e < ECOLS; ++e) {
+            sum[e].hi += __ldcg(&a.part_hi[at + 32 * e]);
+            sum[e].tail += __ldcg(&a.part_tail[at + 32 * e]);
+          }
+        }
+      }
       // Normalise and store, eight columns per step: a rolled loop that moves
       // the remaining sums down the register array (unrolled over 32 columns the
       // code ran at the rate of its instruction fetches).
@@ -601,7 +654,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
       const int n0 = nt * TN + c0;
       const int em = (mlive ? row_scale(a.ea[m - a.m0]) : 0) + a.alpha_exp - 49;
       const int en = row_scale(a.eb[n0 + lane]);
-      const unsigned long long off = kMagicSum * (unsigned long long)np;
       double* dst = a.C.p + (m / a.C.rdiv) * a.C.rs_hi + (m % a.C.rdiv) * a.C.rs_lo +
                     (long long)n0 * a.C.cs;
       const bool vec = a.C.cs == 1 && !a.accumulate && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
@@ -613,7 +665,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
         for (int e = 0; e < 8; ++e) {
           bool x;
           r[e] = __longlong_as_double((long long)finish_sum(
-              (long long)(sum[e].hi - off), sum[e].tail,
+              (long long)sum[e].hi, sum[e].tail,
               em + __shfl_sync(0xffffffffu, en, c + e), a.sign, &x));
           odd |= x ? 1u << e : 0u;
         }
@@ -622,7 +674,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
           for (int e = 0; e < 8; ++e) {
             const int sh = em + __shfl_sync(0xffffffffu, en, c + e);
             if (odd >> e & 1)
-              r[e] = finish_slow((long long)(sum[e].hi - off), sum[e].tail, sh, a.sign);
+              r[e] = finish_slow((long long)sum[e].hi, sum[e].tail, sh, a.sign);
           }
         }
         if (a.scaled) {
@@ -689,6 +741,34 @@ int slice_operand(corr_context* c, const MatView& v, long long r0, int rows, int
 
 }  // namespace
 
+// Parts of each tile's K blocks: few tiles (or a last wave that is nearly
+// empty) leave SMs idle, so the tiles of one launch may be split over K.  The
+// cheapest number of parts, counting a K block of 2304 tensor clocks, 3000 for
+// taking a pass's sums out of TMEM, and for split tiles about 6000 more for the
+// exchange through L2.  715^3 (72 tiles): 30 us with two parts, 42 us whole.
+constexpr int kSplitSms = 152;
+constexpr int kMaxSplit = 16;
+constexpr long long kMaxSplitUnits = 2 * kSplitSms;
+static int k_parts(long long tiles, int nkb) {
+  int best = 1;
+  double cost = 0.0;
+  for (int s = 1; s <= kMaxSplit && s <= nkb; ++s) {
+    if (s > 1 && tiles * s > kMaxSplitUnits) break;
+    const int kper = ceil_div(nkb, s);
+    const double waves = (double)((tiles * s + kSplitSms - 1) / kSplitSms);
+    const double t = waves * (kper * 2304.0 + 3000.0 * ceil_div(kper, PASS_KB)) +
+                     (s > 1 ? 6000.0 + 600.0 * s : 0.0);
+    if (s == 1 || t < 0.95 * cost) {
+      cost = t;
+      best = s;
+    }
+  }
+  return best;
+}
+// Sums and tickets of any split launch: 30 MB, part of every workspace (smaller
+// products than the one a caller sized its workspace for may split further).
+constexpr size_t kSplitBytes = (size_t)kMaxSplitUnits * TM * TN * 12 + kMaxSplitUnits * EWARPS * 4;
+
 // Rows of a launch for K (padded) of kp: a multiple of TM.
 static int row_chunk(int M, size_t kp) {
   const size_t fit = kRowPlaneBytes / (kp * DS * 2) / TM * TM;
@@ -700,7 +780,7 @@ size_t dgemm_tc_workspace(int M, int N, int K) {
   const size_t kp = (size_t)ceil_div(std::min(std::max(K, 1), KCHUNK), DKB) * DKB;
   const size_t mp = row_chunk(M, kp);
   return align256(mp * kp * DS * 2) + align256(np * kp * DS * 2) + align256(mp * 4) +
-         align256(np * 4);
+         align256(np * 4) + align256(kSplitBytes);
 }
 
 size_t dgemm_tc_columns_bytes(int rows, int K) {
@@ -739,6 +819,7 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
   uint16_t* Bw = reinterpret_cast<uint16_t*>(w);
   if (!g.pre) w += align256((size_t)np * kp * DS * 2);
   int* ebw = reinterpret_cast<int*>(w);
+  if (!g.pre) w += align256((size_t)np * 4);
   static bool attr[64] = {};
   if (c->device < 0 || c->device >= 64 || !attr[c->device]) {
     CORR_CUDA(cudaFuncSetAttribute(dgemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -792,7 +873,15 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
       a.a_lower = g.a_lower ? 1 : 0;
       a.k0 = k0;
       a.accumulate = (g.accumulate || p > 0) ? 1 : 0;
-      a.total = (long long)mtn * ntn;
+      const long long tiles = (long long)mtn * ntn;
+      a.nsplit = mp >= g.M ? k_parts(tiles, nkb) : 1;
+      a.kper = ceil_div(nkb, a.nsplit);
+      a.part_hi = reinterpret_cast<unsigned long long*>(w);
+      a.part_tail = reinterpret_cast<float*>(a.part_hi + kMaxSplitUnits * TM * TN);
+      a.ticket = reinterpret_cast<unsigned*>(a.part_tail + kMaxSplitUnits * TM * TN);
+      if (a.nsplit > 1)
+        CORR_CUDA(cudaMemsetAsync(a.ticket, 0, (size_t)tiles * EWARPS * 4, c->stream));
+      a.total = tiles * a.nsplit;
       const int grid = (int)std::min<long long>(a.total, c->sms);
       dgemm_tc_kernel<<<grid, NTHREADS, kDgSmem, c->stream>>>(a, &c->dres->status);
       CORR_CUDA(cudaGetLastError());

@@ -85,3 +85,21 @@ def test_misaligned_device_operands(ctx):
     B = torch.from_numpy(r.standard_normal((77, 40))).cuda()
     C = ctx.dgemm(A, B, tensor_cores=True)
     _check(C.cpu().numpy(), A.cpu().numpy(), B.cpu().numpy())
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (128, 64, 64), (129, 65, 200), (100, 64, 2048), (256, 256, 500), (700, 700, 700),
+    (700, 260, 1030), (1300, 900, 33), (128, 64, 4099),
+])
+def test_tiles_split_over_k(ctx, m, n, k):
+    """Few tiles: each is summed by several CTAs.  Same bound, the same bits on
+    every run, and the same integers whatever part arrives last."""
+    import torch
+
+    r = O.rng(m + n + 2 * k)
+    A, B = r.standard_normal((m, k)), r.standard_normal((k, n))
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    C = ctx.dgemm(dA, dB, tensor_cores=True)
+    _check(C.cpu().numpy(), A, B, extra=(k - 1) // 2048)
+    for _ in range(5):
+        assert torch.equal(ctx.dgemm(dA, dB, tensor_cores=True), C)
