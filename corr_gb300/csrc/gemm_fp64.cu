@@ -178,61 +178,94 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ CU
   }
 }
 
-// Products with few or mostly padded 64 x 64 tiles: 16 x 16 tiles on 64
-// threads, 2 x 2 elements each, plain FP64 FMAs, bounds-checked loads.  The
-// FP64 pipe (two FMAs per clock per SM, DMMA included) bounds every tile shape
-// alike, so what counts is how many FMAs the busiest SM executes: a 64 x 64
-// tile costs 4096 per k however little of it is live.  24 x 24 x 24: 6.0 us
-// (40 us in one 64 x 64 tile); 13824 x 24 x 24: 22 us (77 us).
-constexpr int SBM = 16, SBK = 32;
+// Products with few or mostly padded 64 x 64 tiles: T x T tiles (16 or 8) on 64
+// threads, 2 x 2 elements or one each, plain FP64 FMAs, bounds-checked loads of
+// the next 32 of K while the present ones are used.  The FP64 pipe (two FMAs per
+// clock per SM, DMMA included) bounds every tile shape alike, so what counts is
+// how many FMAs the busiest SM executes: a 64 x 64 tile costs 4096 per k however
+// little of it is live.  24 x 24 x 24: 2.4 us (40 us in one 64 x 64 tile, 6.0 us
+// in 16 x 16 tiles); 64^3 4.5 us (12.6 us in 16 x 16 tiles); 13824 x 24 x 24:
+// 22 us (77 us).
+constexpr int SBK = 32;
 
-template <int TA, int TB>
+template <int T, int TA, int TB>
 __global__ void __launch_bounds__(64) gemm_f64_small_kernel(GemmF64 g) {
-  __shared__ double sa[SBK][SBM + 1], sb[SBK][SBM + 1];
+  constexpr int E = T / 8;             // elements of a thread along each dimension
+  constexpr int L = T * SBK / 64;      // loads of a thread per operand
+  __shared__ double sa[SBK][T + 1], sb[SBK][T + 1];
   const int tid = threadIdx.x;
-  const int m0 = blockIdx.x * SBM, n0 = blockIdx.y * SBM, bz = blockIdx.z;
+  const int m0 = blockIdx.x * T, n0 = blockIdx.y * T, bz = blockIdx.z;
   const double* A = g.A + (long long)bz * g.sa;
   const double* B = g.B + (long long)bz * g.sb;
-  const int tm = (tid >> 3) * 2, tn = (tid & 7) * 2;
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-  for (int k0 = 0; k0 < g.K; k0 += SBK) {
+  const int tm = (tid >> 3) * E, tn = (tid & 7) * E;
+  double acc[E][E];
 #pragma unroll
-    for (int e = 0; e < SBM * SBK / 64; ++e) {
+  for (int i = 0; i < E; ++i)
+#pragma unroll
+    for (int j = 0; j < E; ++j) acc[i][j] = 0.0;
+  double ra[L], rb[L];
+  auto load = [&](int k0) {  // consecutive threads along the operand's contiguous dimension
+#pragma unroll
+    for (int e = 0; e < L; ++e) {
       const int idx = tid + 64 * e;
-      // consecutive threads along the operand's contiguous dimension
-      const int ra = TA == 0 ? idx / SBK : idx % SBM, ka = TA == 0 ? idx % SBK : idx / SBM;
-      const int m = m0 + ra, k = k0 + ka;
-      sa[ka][ra] = m < g.M && k < g.K
-                       ? (TA == 0 ? A[(long long)m * g.lda + k] : A[(long long)k * g.lda + m])
-                       : 0.0;
-      const int rb = TB == 0 ? idx % SBM : idx / SBK, kb = TB == 0 ? idx / SBM : idx % SBK;
-      const int n = n0 + rb, kk = k0 + kb;
-      sb[kb][rb] = n < g.N && kk < g.K
-                       ? (TB == 0 ? B[(long long)kk * g.ldb + n] : B[(long long)n * g.ldb + kk])
-                       : 0.0;
+      const int m = m0 + (TA == 0 ? idx / SBK : idx % T), k = k0 + (TA == 0 ? idx % SBK : idx / T);
+      ra[e] = m < g.M && k < g.K
+                  ? (TA == 0 ? A[(long long)m * g.lda + k] : A[(long long)k * g.lda + m])
+                  : 0.0;
+      const int n = n0 + (TB == 0 ? idx % T : idx / SBK), q = k0 + (TB == 0 ? idx / T : idx % SBK);
+      rb[e] = n < g.N && q < g.K
+                  ? (TB == 0 ? B[(long long)q * g.ldb + n] : B[(long long)n * g.ldb + q])
+                  : 0.0;
+    }
+  };
+  load(0);
+  for (int k0 = 0; k0 < g.K; k0 += SBK) {
+    if (k0) __syncthreads();
+#pragma unroll
+    for (int e = 0; e < L; ++e) {
+      const int idx = tid + 64 * e;
+      sa[TA == 0 ? idx % SBK : idx / T][TA == 0 ? idx / SBK : idx % T] = ra[e];
+      sb[TB == 0 ? idx / T : idx % SBK][TB == 0 ? idx % T : idx / SBK] = rb[e];
     }
     __syncthreads();
+    if (k0 + SBK < g.K) load(k0 + SBK);
     const int ke = min(SBK, g.K - k0);
+#pragma unroll 4
     for (int k = 0; k < ke; ++k) {
-      const double a0 = sa[k][tm], a1 = sa[k][tm + 1], b0 = sb[k][tn], b1 = sb[k][tn + 1];
-      acc[0][0] = fma(a0, b0, acc[0][0]);
-      acc[0][1] = fma(a0, b1, acc[0][1]);
-      acc[1][0] = fma(a1, b0, acc[1][0]);
-      acc[1][1] = fma(a1, b1, acc[1][1]);
+      double a[E], b[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        a[i] = sa[k][tm + i];
+        b[i] = sb[k][tn + i];
+      }
+#pragma unroll
+      for (int i = 0; i < E; ++i)
+#pragma unroll
+        for (int j = 0; j < E; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
     }
-    __syncthreads();
   }
   double* C = g.C + (long long)bz * g.sc;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < E; ++i)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < E; ++j) {
       const int m = m0 + tm + i, n = n0 + tn + j;
       if (m >= g.M || n >= g.N) continue;
       double* c = C + (long long)m * g.ldc + n;
       const double v = g.alpha * acc[i][j];
       *c = g.beta == 0.0 ? v : v + g.beta * (*c);
     }
+}
+
+template <int T>
+int launch_small(const GemmF64& g, cudaStream_t s) {
+  const dim3 grid((g.M + T - 1) / T, (g.N + T - 1) / T, g.batch);
+  if (g.ta == 0 && g.tb == 0) gemm_f64_small_kernel<T, 0, 0><<<grid, 64, 0, s>>>(g);
+  else if (g.ta == 0) gemm_f64_small_kernel<T, 0, 1><<<grid, 64, 0, s>>>(g);
+  else if (g.tb == 0) gemm_f64_small_kernel<T, 1, 0><<<grid, 64, 0, s>>>(g);
+  else gemm_f64_small_kernel<T, 1, 1><<<grid, 64, 0, s>>>(g);
+  CORR_CUDA(cudaGetLastError());
+  return CORR_OK;
 }
 
 // FMAs on the busiest of the GPU's SMs for tiles of t x t over K steps of kb.
@@ -250,18 +283,12 @@ bool aligned16(const void* p, long long ld) {
 
 int gemm_f64(const GemmF64& g, int* status, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return CORR_OK;
-  // small tiles where they leave the busiest SM less than half the work (their
-  // loads are not pipelined, so a smaller margin is not worth taking)
-  const dim3 sgrid((g.M + SBM - 1) / SBM, (g.N + SBM - 1) / SBM, g.batch);
-  if (2.0 * busiest_sm(g, SBM, 1) <= busiest_sm(g, BM, BK) && sgrid.y <= 65535 &&
-      sgrid.z <= 65535) {
-    if (g.ta == 0 && g.tb == 0) gemm_f64_small_kernel<0, 0><<<sgrid, 64, 0, s>>>(g);
-    else if (g.ta == 0) gemm_f64_small_kernel<0, 1><<<sgrid, 64, 0, s>>>(g);
-    else if (g.tb == 0) gemm_f64_small_kernel<1, 0><<<sgrid, 64, 0, s>>>(g);
-    else gemm_f64_small_kernel<1, 1><<<sgrid, 64, 0, s>>>(g);
-    CORR_CUDA(cudaGetLastError());
-    return CORR_OK;
-  }
+  // small tiles where they leave the busiest SM less than half of the 64 x 64
+  // tiles' work (their loads go through registers, so a smaller margin is not
+  // worth taking); 8 x 8 where they halve it again
+  const double w64 = busiest_sm(g, BM, BK), w16 = busiest_sm(g, 16, 1), w8 = busiest_sm(g, 8, 1);
+  const bool fits = g.batch <= 65535 && (g.N + 7) / 8 <= 65535;
+  if (fits && 2.0 * w16 <= w64) return 2.0 * w8 <= w16 ? launch_small<8>(g, s) : launch_small<16>(g, s);
   CUtensorMap ta{}, tb{};
   // TMA needs 16-byte aligned base/leading dimension and batch strides
   bool tmaA = aligned16(g.A, g.lda) && (g.sa * 8) % 16 == 0 && g.K > 0;

@@ -30,13 +30,12 @@ int gemm_f64(const GemmF64& g, int* status, cudaStream_t s);
 // kStatusNeedFp64.
 size_t gemm_plain_workspace(const corr_context* c, long long M, long long N, long long K);
 int gemm_plain(corr_context* c, const GemmF64& g, void* ws);
-// The rule: from about 1e7 multiply-adds on, where the FP64 pipe takes 17 us at
-// its full rate of 5.9e5 per us, the slicing and one tile of the digit GEMM
-// (about 25 us in all, three launches) are the shorter way; 13824 x 24 x 24 is
-// 22 us against 30 us, 256^3 47 us against 47 us, 300 x 300 x 300 and larger
-// the digit GEMM's.
+// The rule: from 1e7 multiply-adds on, where the FP64 pipe takes 17 us at its
+// full rate of 5.9e5 per us, the slicing (three launches, about 10 us) and one
+// round of digit-GEMM tiles are the shorter way: 200^3 takes 34 us on either,
+// 256^3 42 us against 34 us, 128^3 8 us against 28 us.
 inline bool digits_pay(const corr_context* c, long long M, long long N, long long K) {
-  return !c->fp64_strict && (double)M * N * K >= 2e7 && M <= 0x7fffff00LL && N <= 0x7fffff00LL;
+  return !c->fp64_strict && (double)M * N * K >= 1e7 && M <= 0x7fffff00LL && N <= 0x7fffff00LL;
 }
 
 inline GemmF64 gemm_args(const double* A, const double* B, double* C, int M, int N, int K,

@@ -30,7 +30,7 @@ def _same_energy(a, b, tol=1e-12):
         assert abs(x - y) <= tol * max(abs(y), abs(b.e_total)), (x, y)
 
 
-# (o v)^2 naux around 3e7; nvir around the 32-wide panel tiles and the 64-wide
+# (o v)^2 naux around the rule; nvir around the 32-wide panel tiles and the 64-wide
 # column tiles; two panels of 512 MiB in the last
 @pytest.mark.parametrize("o,v,x", [
     (10, 100, 29), (10, 100, 30), (10, 100, 31), (1, 640, 120), (64, 10, 90), (33, 31, 40),
