@@ -423,8 +423,8 @@ struct StreamSwap {
 
 int chol_factor_device(corr_context* c, void* ws, const double* J, int m, double shift,
                        double** Lm_out, double** Linv_out, bool* ok, void* tc_ws);
-int chol_inverse_device(corr_context* c, const double* Lm, const double* Linv, int m, double* X,
-                        double* T, void* tc_ws);
+int chol_factor_inverse_device(corr_context* c, void* ws, const double* J, int m, double shift,
+                               double* X, double* T, double** Lm_out, bool* ok, void* tc_ws);
 int chol_norm_one_inf(corr_context* c, void* scratch, const double* X, int m, double* out);
 int chol_solve_device(corr_context* c, const double* Lm, const double* Linv, int m, double* P,
                       long long ncols, double* out);
@@ -646,9 +646,8 @@ int corr_rimp2_energy_from_3index(corr_context* c, int nroe, int nroao, int naux
         // factored (chol.cu); without a certificate, J^-1/2 with the cutoff.
         CORR_TRY(chol_norm_inf(c, jm, d_j, X, &jnorm));
         if (jnorm > 0.0)
-          CORR_TRY(chol_factor_device(c, jws, d_j, X, 0.0, &Lm, &Linv, &factored, mws));
+          CORR_TRY(chol_factor_inverse_device(c, jws, d_j, X, 0.0, W, T, &Lm, &factored, mws));
         if (factored) {
-          CORR_TRY(chol_inverse_device(c, Lm, Linv, X, W, T, mws));
           double n1inf = 0.0;
           CORR_TRY(chol_norm_one_inf(c, jm, W, X, &n1inf));
           bool certified = n1inf > 0.0 && 1.0 / n1inf > 2.0 * 10.0 * tol * jnorm;
