@@ -160,6 +160,13 @@ __device__ __forceinline__ void store_chunk(const double (&x)[8], int er, uint16
         make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
 }
 
+// The arrival counters of a product whose tiles are split over K start at zero;
+// the slicing of its row operand, just ahead of it, clears them.
+__device__ __forceinline__ void clear_tickets(unsigned* zero, int n) {
+  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x)
+    zero[x] = 0u;
+}
+
 // Slicing of an operand whose k are adjacent in memory: `lpr` lanes (a power
 // of two) take one row, find its exponent and write its digit planes in one
 // launch; the second read of the row comes from L1/L2.  Bound by HBM (8 bytes
@@ -171,7 +178,9 @@ __global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, long long r0
                                                          int kn, int nkb, int lpr,
                                                          int* __restrict__ e,
                                                          uint16_t* __restrict__ out,
-                                                         int* __restrict__ status) {
+                                                         int* __restrict__ status,
+                                                         unsigned* __restrict__ zero, int nzero) {
+  clear_tickets(zero, nzero);
   const int nch = nkb * (DKB / 8);
   const int lane = threadIdx.x & 31, sub = lane & (lpr - 1), per = 32 / lpr;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -268,7 +277,9 @@ __global__ void __launch_bounds__(256) slice_kcol_kernel(MatView v, long long r0
                                                          int rows_pad, int k0,
                                                          int kn, int nkb,
                                                          const int* __restrict__ e,
-                                                         uint16_t* __restrict__ out) {
+                                                         uint16_t* __restrict__ out,
+                                                         unsigned* __restrict__ zero, int nzero) {
+  clear_tickets(zero, nzero);
   const int nc2 = nkb * (DKB / 16);
   const long long total = (long long)rows_pad * nc2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
@@ -715,7 +726,7 @@ size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 template <int TR>
 int slice_operand(corr_context* c, const MatView& v, long long r0, int rows, int rows_pad, int k0, int kn,
-                  int nkb, int* e, uint16_t* out) {
+                  int nkb, int* e, uint16_t* out, unsigned* zero = nullptr, int nzero = 0) {
   const int cap = c->sms * 16;
   int* status = c->digit_guard ? &c->dres->status : nullptr;
   if (v.ks == 1) {  // k contiguous
@@ -723,7 +734,7 @@ int slice_operand(corr_context* c, const MatView& v, long long r0, int rows, int
     while (lpr < 32 && lpr < nkb * (DKB / 8)) lpr *= 2;
     const int grid = std::min(ceil_div((long long)rows_pad * lpr, 256), cap);
     slice_krow_kernel<TR><<<grid, 256, 0, c->stream>>>(v, r0, rows, rows_pad, k0, kn, nkb, lpr, e,
-                                                       out, status);
+                                                       out, status, zero, nzero);
     CORR_CUDA(cudaGetLastError());
     c->launches += 1;
     return CORR_OK;
@@ -733,7 +744,8 @@ int slice_operand(corr_context* c, const MatView& v, long long r0, int rows, int
   col_exponent_kernel<<<eg, 256, 0, c->stream>>>(v, r0, rows, k0, kn, e, status);
   CORR_CUDA(cudaGetLastError());
   const int grid = std::min(ceil_div((long long)rows_pad * nkb * (DKB / 16), 256), cap);
-  slice_kcol_kernel<TR><<<grid, 256, 0, c->stream>>>(v, r0, rows, rows_pad, k0, kn, nkb, e, out);
+  slice_kcol_kernel<TR><<<grid, 256, 0, c->stream>>>(v, r0, rows, rows_pad, k0, kn, nkb, e, out, zero,
+                                                      nzero);
   CORR_CUDA(cudaGetLastError());
   c->launches += 2;
   return CORR_OK;
@@ -846,8 +858,14 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
     }
     for (int m0 = 0; m0 < g.M; m0 += mp) {
       const int rows = std::min(mp, g.M - m0), mtn = ceil_div(rows, TM);
+      const long long tiles = (long long)mtn * ntn;
+      const int parts = mp >= g.M && kn > 0 ? k_parts(tiles, nkb) : 1;
+      unsigned long long* part_hi = reinterpret_cast<unsigned long long*>(w);
+      float* part_tail = reinterpret_cast<float*>(part_hi + kMaxSplitUnits * TM * TN);
+      unsigned* ticket = reinterpret_cast<unsigned*>(part_tail + kMaxSplitUnits * TM * TN);
       if (kn > 0) {
-        CORR_TRY(slice_operand<TM>(c, g.A, m0, rows, mtn * TM, k0, kn, nkb, ea, Ad));
+        CORR_TRY(slice_operand<TM>(c, g.A, m0, rows, mtn * TM, k0, kn, nkb, ea, Ad, ticket,
+                                   parts > 1 ? (int)tiles * EWARPS : 0));
       } else {
         CORR_CUDA(cudaMemsetAsync(Ad, 0, (size_t)mp * kp * DS * 2, c->stream));
         CORR_CUDA(cudaMemsetAsync(ea, 0, (size_t)mp * 4, c->stream));
@@ -873,14 +891,11 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
       a.a_lower = g.a_lower ? 1 : 0;
       a.k0 = k0;
       a.accumulate = (g.accumulate || p > 0) ? 1 : 0;
-      const long long tiles = (long long)mtn * ntn;
-      a.nsplit = mp >= g.M ? k_parts(tiles, nkb) : 1;
-      a.kper = ceil_div(nkb, a.nsplit);
-      a.part_hi = reinterpret_cast<unsigned long long*>(w);
-      a.part_tail = reinterpret_cast<float*>(a.part_hi + kMaxSplitUnits * TM * TN);
-      a.ticket = reinterpret_cast<unsigned*>(a.part_tail + kMaxSplitUnits * TM * TN);
-      if (a.nsplit > 1)
-        CORR_CUDA(cudaMemsetAsync(a.ticket, 0, (size_t)tiles * EWARPS * 4, c->stream));
+      a.nsplit = parts;
+      a.kper = ceil_div(nkb, parts);
+      a.part_hi = part_hi;
+      a.part_tail = part_tail;
+      a.ticket = ticket;
       a.total = tiles * a.nsplit;
       const int grid = (int)std::min<long long>(a.total, c->sms);
       dgemm_tc_kernel<<<grid, NTHREADS, kDgSmem, c->stream>>>(a, &c->dres->status);

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ CU
 // how many FMAs the busiest SM executes: a 64 x 64 tile costs 4096 per k however
 // little of it is live.  24 x 24 x 24: 2.4 us (40 us in one 64 x 64 tile, 6.0 us
 // in 16 x 16 tiles); 64^3 4.5 us (12.6 us in 16 x 16 tiles); 13824 x 24 x 24:
-// 22 us (77 us).
+// 17 us (77 us; 22 us in 16 x 16 tiles).
 constexpr int SBK = 32;
 
 template <int T, int TA, int TB>
@@ -285,10 +285,10 @@ int gemm_f64(const GemmF64& g, int* status, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return CORR_OK;
   // small tiles where they leave the busiest SM less than half of the 64 x 64
   // tiles' work (their loads go through registers, so a smaller margin is not
-  // worth taking); 8 x 8 where they halve it again
+  // worth taking); 8 x 8 where they save another sixth
   const double w64 = busiest_sm(g, BM, BK), w16 = busiest_sm(g, 16, 1), w8 = busiest_sm(g, 8, 1);
   const bool fits = g.batch <= 65535 && (g.N + 7) / 8 <= 65535;
-  if (fits && 2.0 * w16 <= w64) return 2.0 * w8 <= w16 ? launch_small<8>(g, s) : launch_small<16>(g, s);
+  if (fits && 2.0 * w16 <= w64) return 1.2 * w8 <= w16 ? launch_small<8>(g, s) : launch_small<16>(g, s);
   CUtensorMap ta{}, tb{};
   // TMA needs 16-byte aligned base/leading dimension and batch strides
   bool tmaA = aligned16(g.A, g.lda) && (g.sa * 8) % 16 == 0 && g.K > 0;

@@ -32,7 +32,7 @@ size_t gemm_plain_workspace(const corr_context* c, long long M, long long N, lon
 int gemm_plain(corr_context* c, const GemmF64& g, void* ws);
 // The rule: from 1e7 multiply-adds on, where the FP64 pipe takes 17 us at its
 // full rate of 5.9e5 per us, the slicing (three launches, about 10 us) and one
-// round of digit-GEMM tiles are the shorter way: 200^3 takes 34 us on either,
+// round of digit-GEMM tiles are the shorter way: 200^3 takes 18 us against 33 us,
 // 256^3 42 us against 34 us, 128^3 8 us against 28 us.
 inline bool digits_pay(const corr_context* c, long long M, long long N, long long K) {
   return !c->fp64_strict && (double)M * N * K >= 1e7 && M <= 0x7fffff00LL && N <= 0x7fffff00LL;

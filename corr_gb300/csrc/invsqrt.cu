@@ -18,7 +18,9 @@
 // iteration), so l_k+1 = p(a_k l_k) grows by ~2.6 per step instead of 1.5,
 // from l_0 = (t / c)^1/2.  Then unscaled steps until max|Z Y - I| stops
 // falling below 1e-14 (quadratic convergence).  Products of symmetric
-// iterates are symmetric up to rounding; the result is symmetrised.
+// iterates are symmetric up to rounding; the result is symmetrised.  (Reading a
+// factor's rows in place of its columns would save two slicing launches a
+// product, but the rounding asymmetry then grows and the iteration fails.)
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -69,6 +71,14 @@ __global__ void ns_init_kernel(const double* __restrict__ J, int m, double rc,
     Y[x] = J[x] * rc;
     Z[x] = (x / m) == (x % m) ? 1.0 : 0.0;
   }
+}
+
+// out = a x
+__global__ void scale_kernel(const double* __restrict__ x, long long n, double a,
+                             double* __restrict__ out) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x)
+    out[k] = a * x[k];
 }
 
 // out = (Z + Z^T) / (2 sqrt(c)); sum of squares of J for the Frobenius norm
@@ -323,9 +333,10 @@ int ri_inv_sqrt_ns(corr_context* c, void* ws, const double* J, int m, double tol
   for (int it = 0; it < 60; ++it) {
     const bool scaled = l < 0.999;
     const double a2 = scaled ? 3.0 / (1.0 + l + l * l) : 1.0, a = std::sqrt(a2);
-    CORR_TRY(gemm(Z, Y, P, 1.0));
+    const bool first = it == 0;  // Z = I: Z Y = Y, and a T Z = a T below
+    if (!first) CORR_TRY(gemm(Z, Y, P, 1.0));
     CORR_CUDA(cudaMemsetAsync(derr, 0, 8, s));
-    ns_step_kernel<<<grid, 256, 0, s>>>(P, m, a2, T, derr);
+    ns_step_kernel<<<grid, 256, 0, s>>>(first ? Y : P, m, a2, T, derr);
     CORR_CUDA(cudaGetLastError());
     c->launches += 1;
     double err = 0.0;
@@ -344,8 +355,14 @@ int ri_inv_sqrt_ns(corr_context* c, void* ws, const double* J, int m, double tol
     // Y <- a Y T, Z <- a T Z (into P, then swap)
     CORR_TRY(gemm(Y, T, P, a));
     std::swap(Y, P);
-    CORR_TRY(gemm(T, Z, P, a));
-    std::swap(Z, P);
+    if (first) {
+      scale_kernel<<<grid, 256, 0, s>>>(T, (long long)mm, a, Z);
+      CORR_CUDA(cudaGetLastError());
+      c->launches += 1;
+    } else {
+      CORR_TRY(gemm(T, Z, P, a));
+      std::swap(Z, P);
+    }
     if (scaled) {
       const double x = a * l;
       l = std::min(1.0, 0.5 * x * (3.0 - x * x));
