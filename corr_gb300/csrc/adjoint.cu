@@ -272,8 +272,8 @@ int rimp2_gradient_tc(corr_context* c, Carver& w, int o, int v, int X, const dou
     const long long r0 = (long long)i0 * v, r1 = (long long)(i0 + ni) * v;
     PanelView pv;
     CORR_TRY(panel_product(c, o, v, X, bia, cols, i0, ni, panel, dws, &pv));
-    CORR_TRY(launch_panel(c, pv, eps, deps, part + 2 * np, true));
-    np += (long long)ni * (o - i0);
+    CORR_TRY(launch_panel(c, pv, eps, deps, part + 2 * np, p.split, true));
+    np += (long long)ni * (o - i0) * p.split;
     DgemmTc d;
     d.A = mat_view(bia + r0, R, 1);                        // rows Q, over (j, b)
     d.B = mat_view(panel + (r0 - pv.col0), pv.ld, 1);      // rows (i, a), over (j, b)

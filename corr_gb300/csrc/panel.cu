@@ -35,8 +35,10 @@ __device__ __forceinline__ double recip64(double d) {
   return fma(r, fma(e, e, e), r);
 }
 
-// One CTA per (i, j) block of the panel, 32 x 32 tile pairs (A <= B): a thread
-// owns the pair (a, b), (b, a), the transposed tile comes (and goes back)
+// CTAs of an (i, j) block of the panel (blockIdx.x) share its columns of 32 x 32
+// tile pairs (A <= B, column B to blockIdx.y): with one CTA per block the 276
+// blocks of 23 occupied orbitals left most of the GPU waiting for one another's
+// loads (energy nocc=23 nvir=211: 187 us against 278 us).  A thread owns the pair (a, b), (b, a), the transposed tile comes (and goes back)
 // through shared memory, so every access to the panel is coalesced.  Diagonal
 // tiles see each pair from both sides at weight 1/2.
 //
@@ -59,8 +61,9 @@ __global__ void __launch_bounds__(256) panel_kernel(PanelView pv, const double* 
   const int il = blockIdx.x / nj, i = pv.i0 + il, j = pv.i0 + blockIdx.x % nj;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const bool count = j >= i;
+  const long long slot = (long long)blockIdx.x * gridDim.y + blockIdx.y;
   if (!GRAD && !count) {
-    if (threadIdx.x < 2) part[2 * (long long)blockIdx.x + threadIdx.x] = 0.0;
+    if (threadIdx.x < 2) part[2 * slot + threadIdx.x] = 0.0;
     return;
   }
   if (GRAD) {
@@ -71,7 +74,7 @@ __global__ void __launch_bounds__(256) panel_kernel(PanelView pv, const double* 
   const double eij = eps[i] + eps[j];
   const int nt = (v + PT - 1) / PT;
   double s0 = 0.0, s1 = 0.0;  // energy: os, ss; gradient: E, sum of W
-  for (int tB = 0; tB < nt; ++tB) {
+  for (int tB = blockIdx.y; tB < nt; tB += gridDim.y) {
     const int b = tB * PT + tx;
     const double eb = b < v ? eps[o + b] : 0.0;
     double wcol = 0.0;
@@ -176,13 +179,13 @@ __global__ void __launch_bounds__(256) panel_kernel(PanelView pv, const double* 
         atomicAdd(&deps[i], -wij * ws);
         atomicAdd(&deps[j], -wij * ws);
       }
-      part[2 * (long long)blockIdx.x] = count ? wij * es : 0.0;
-      part[2 * (long long)blockIdx.x + 1] = 0.0;
+      part[2 * slot] = count ? wij * es : 0.0;
+      part[2 * slot + 1] = 0.0;
     }
   } else if (threadIdx.x < 2) {
     double t = 0.0;
     for (int k = 0; k < 8; ++k) t += red[threadIdx.x][k];
-    part[2 * (long long)blockIdx.x + threadIdx.x] = -wij * t;
+    part[2 * slot + threadIdx.x] = -wij * t;
   }
 }
 
@@ -196,7 +199,10 @@ PanelPlan panel_plan(int o, int v, int X, size_t budget) {
   p.col_bytes = dgemm_tc_columns_bytes(o * v, X);
   long long n = 0;
   for (int i0 = 0; i0 < o; i0 += p.ni) n += (long long)std::min(p.ni, o - i0) * (o - i0);
-  p.partials = n;
+  // CTAs per (i, j) block: one per column of tiles while that is a few million
+  const int nt = (v + PT - 1) / PT;
+  p.split = n * nt <= (1ll << 22) && nt <= 65535 ? nt : 1;
+  p.partials = n * p.split;
   return p;
 }
 
@@ -226,8 +232,8 @@ int panel_product(corr_context* c, int o, int v, int X, const double* bia, const
 }
 
 int launch_panel(corr_context* c, const PanelView& pv, const double* eps, double* deps,
-                 double* part, bool grad) {
-  const int grid = pv.ni * (pv.o - pv.i0);
+                 double* part, int split, bool grad) {
+  const dim3 grid((unsigned)(pv.ni * (pv.o - pv.i0)), (unsigned)split);
   if (grad)
     panel_kernel<true><<<grid, 256, (size_t)pv.v * 8, c->stream>>>(pv, eps, deps, part);
   else
@@ -265,8 +271,8 @@ int energy_from_panels(corr_context* c, Carver& w, int o, int v, int X, const do
     const int ni = std::min(p.ni, o - i0);
     PanelView pv;
     CORR_TRY(panel_product(c, o, v, X, bia, cols, i0, ni, panel, dws, &pv));
-    CORR_TRY(launch_panel(c, pv, eps, nullptr, part + 2 * np, false));
-    np += (long long)ni * (o - i0);
+    CORR_TRY(launch_panel(c, pv, eps, nullptr, part + 2 * np, p.split, false));
+    np += (long long)ni * (o - i0) * p.split;
   }
   CORR_CUDA(cudaMemsetAsync(ticket, 0, 16, c->stream));
   const int nr = launch_unit_reduce(part, (int)np, nullptr, out_e, scratch, ticket, c->stream);

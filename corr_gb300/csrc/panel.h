@@ -19,7 +19,7 @@ struct PanelView {
 // one orbital), the column operand's digit planes, and the partials of all
 // launch_panel calls.
 struct PanelPlan {
-  int ni;
+  int ni, split;
   size_t panel_bytes, col_bytes;
   long long partials;
 };
@@ -31,9 +31,10 @@ PanelPlan panel_plan(int o, int v, int X, size_t budget);
 int panel_product(corr_context* c, int o, int v, int X, const double* bia, const DgColumns& cols,
                   int i0, int ni, double* panel, void* dws, PanelView* pv);
 // Energy partials ({E_OS, E_SS} per CTA), or with grad the elements replaced by
-// the adjoint G, W added to deps and {E, 0} partials.  ni (o - i0) partials.
+// the adjoint G, W added to deps and {E, 0} partials.  split (of the plan): CTAs
+// per (i, j) block; ni (o - i0) split partials.
 int launch_panel(corr_context* c, const PanelView& pv, const double* eps, double* deps,
-                 double* part, bool grad);
+                 double* part, int split, bool grad);
 
 // The plain form's energy: scratch bytes, and the evaluation on device-resident
 // inputs (raises kStatusNeedFp64 for values out of the digit GEMM's range).
