@@ -55,6 +55,7 @@ struct corr_context {
   bool attrs_set = false;  // one-time kernel attributes (kept out of graph capture)
   int fp64_strict = 0;     // 1: the plain form uses the FP64 pipe only (corr_set_fp64_strict)
   bool digit_guard = false;  // a plain-form call is running on the digit GEMM
+  int spare_sms = 0;  // SMs that digit-GEMM launches leave free
   // batched driver
   int batch_order = 1;   // 0 input order, 1 cost-descending
   int batch_stages = 3;

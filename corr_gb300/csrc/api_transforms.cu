@@ -397,7 +397,11 @@ struct SideStream {
   cudaStream_t st = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   int fork(cudaStream_t from) {
-    CORR_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    // highest priority: its kernels are short and dependent, and get the SMs that
+    // the long products of the other stream free first
+    int least = 0, greatest = 0;
+    CORR_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    CORR_CUDA(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, greatest));
     for (cudaEvent_t& e : ev) CORR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CORR_CUDA(cudaEventRecord(ev[0], from));
     CORR_CUDA(cudaStreamWaitEvent(st, ev[0], 0));
@@ -636,7 +640,15 @@ int corr_rimp2_energy_from_3index(corr_context* c, int nroe, int nroao, int naux
       SideStream side;
       CORR_TRY(side.fork(c->stream));
       // (P|ia); (P|mu nu) is symmetric in mu nu
-      CORR_TRY(mo_block_digits(c, X, N, o, d_m, d_p, true, biq, pia, dws));
+      // The products leave 24 of the 152 SMs to the metric: a CTA of the digit
+      // GEMM fills its SM's shared memory for the whole launch, so the dependent
+      // kernels of the factorisation would only run between launches.  20-water
+      // cluster, whole pipeline: 16.3 ms with none left, 15.7 with 2, 14.8 with
+      // 12, 14.4 with 24, 14.7 with 40.
+      c->spare_sms = 24;
+      const int st = mo_block_digits(c, X, N, o, d_m, d_p, true, biq, pia, dws);
+      c->spare_sms = 0;
+      CORR_TRY(st);
       {
         StreamSwap onside(c, side.st);
         // The metric (ri.cc:50-69): one factorisation J = L L^T and W = L^-1

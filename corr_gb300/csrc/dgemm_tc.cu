@@ -897,7 +897,7 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
       a.part_tail = part_tail;
       a.ticket = ticket;
       a.total = tiles * a.nsplit;
-      const int grid = (int)std::min<long long>(a.total, c->sms);
+      const int grid = (int)std::min<long long>(a.total, c->sms - c->spare_sms);
       dgemm_tc_kernel<<<grid, NTHREADS, kDgSmem, c->stream>>>(a, &c->dres->status);
       CORR_CUDA(cudaGetLastError());
       c->launches += 1;
