@@ -194,7 +194,8 @@ int corr_set_energy_tiles(corr_context* ctx, int tiles);
  * (corr_dgemm_tc), and J^-1/2 of a certified metric is computed by
  * Newton-Schulz on it (5e-11 from LAPACK's on the 20-water cluster); inputs
  * outside the digit GEMM's range (not finite, rows of subnormals) repeat the
- * call on the FP64 pipe.  1: every product on the FP64 pipe and J^-1/2 by the
+ * call on the FP64 pipe (corr_calculate_ri expects finite inputs).  1: every
+ * product on the FP64 pipe and J^-1/2 by the
  * eigendecomposition -- IEEE FP64 end to end, many times slower.
  * corr_rimp2_energy_async, the batched calls and corr_rimp2_energy_noalloc run
  * their FP64 form on the FP64 pipe in either mode. */
