@@ -183,9 +183,9 @@ class Context:
         check(self._L.corr_selftest_wait_timeout(self._h, int(limit_ms)))
 
     def set_fp64_strict(self, strict=True):
-        """Plain-form calls (precision "fp64", the transforms and the metric) on
-        the FP64 pipe only (True) or with their large products on the
-        FP64-accurate digit GEMM (False, the default)."""
+        """Plain-form calls on the FP64 pipe only (True), or with the panels of
+        large "fp64" energies, the gradient and the metric on the FP64-accurate
+        digit GEMM (False, the default)."""
         check(self._L.corr_set_fp64_strict(self._h, 1 if strict else 0))
 
     def set_energy_tiles(self, tiles):

@@ -9,7 +9,7 @@
 
 namespace corr {
 int quarter(corr_context* c, const double* in, const double* mos, int N, int crow, int nout,
-            long long M, double* out, void* dws);
+            long long M, double* out);
 int launch_unpack(corr_context* c, int N, long long n, const long long* sc, const double* val,
                   const unsigned short* num, double* eri);
 int launch_canonical(corr_context* c, const double* t, int full, int N, int o, int v,
@@ -17,11 +17,6 @@ int launch_canonical(corr_context* c, const double* t, int full, int N, int o, i
 int canonical_grid(corr_context* c, long long total);
 
 namespace {
-
-// Digit-GEMM workspace of the quarter transforms (the first has the most rows).
-size_t quarter_workspace(const corr_context* c, int N) {
-  return gemm_plain_workspace(c, (long long)N * N * N, N, N);
-}
 
 // Stage the packed ERI list and the MO coefficients, then build (ia|jb) or the
 // full MO tensor into `dst` (device).
@@ -36,7 +31,6 @@ int motrans_device(corr_context* c, Carver& w, int nroe, int N, const double* mo
   void* s_num = w.take((size_t)(nint > 0 ? nint : 1) * 8);
   double* t0 = static_cast<double*>(w.take(n4 * 8));
   double* t1 = static_cast<double*>(w.take(n4 * 8));
-  void* dws = w.take(quarter_workspace(c, N));
   const double* d_mos = static_cast<const double*>(stage_in(c, mos, (size_t)N * N * 8, s_mos));
   const long long* d_sc = static_cast<const long long*>(stage_in(c, sortcount, 32, s_sc));
   const double* d_val = nint > 0 ? static_cast<const double*>(stage_in(c, intval, nint * 8, s_val))
@@ -52,28 +46,24 @@ int motrans_device(corr_context* c, Carver& w, int nroe, int N, const double* mo
   const long long N3 = (long long)N * N * N;
   mark(c, 1);
   if (full) {
-    CORR_TRY(quarter(c, t0, d_mos, N, 0, N, N3, t1, dws));
-    CORR_TRY(quarter(c, t1, d_mos, N, 0, N, N3, t0, dws));
-    CORR_TRY(quarter(c, t0, d_mos, N, 0, N, N3, t1, dws));
-    CORR_TRY(quarter(c, t1, d_mos, N, 0, N, N3, dst, dws));
+    CORR_TRY(quarter(c, t0, d_mos, N, 0, N, N3, t1));
+    CORR_TRY(quarter(c, t1, d_mos, N, 0, N, N3, t0));
+    CORR_TRY(quarter(c, t0, d_mos, N, 0, N, N3, t1));
+    CORR_TRY(quarter(c, t1, d_mos, N, 0, N, N3, dst));
   } else {
-    CORR_TRY(quarter(c, t0, d_mos, N, 0, o, N3, t1, dws));                          // [bcd][i]
-    CORR_TRY(quarter(c, t1, d_mos, N, o, v, (long long)N * N * o, t0, dws));       // [cdi][a]
-    CORR_TRY(quarter(c, t0, d_mos, N, 0, o, (long long)N * o * v, t1, dws));       // [dia][j]
-    CORR_TRY(quarter(c, t1, d_mos, N, o, v, (long long)o * v * o, dst, dws));      // [iaj][b]
+    CORR_TRY(quarter(c, t0, d_mos, N, 0, o, N3, t1));                          // [bcd][i]
+    CORR_TRY(quarter(c, t1, d_mos, N, o, v, (long long)N * N * o, t0));       // [cdi][a]
+    CORR_TRY(quarter(c, t0, d_mos, N, 0, o, (long long)N * o * v, t1));       // [dia][j]
+    CORR_TRY(quarter(c, t1, d_mos, N, o, v, (long long)o * v * o, dst));      // [iaj][b]
   }
   mark(c, 2);
+  c->launches += 4;
   return CORR_OK;
 }
 
 // out[Q][i][a] = sum_(mu nu) C[i][mu] b[Q][mu][nu] C[o+a][nu] through
-// biq[Q][i][nu] (transform_ri, ri.cc:147-172).  `symmetric`: b[Q] is symmetric,
-// so its rows serve as its columns and the first product reads adjacent k.
-size_t mo_block_workspace(const corr_context* c, int X, int N, int o) {
-  if (!digits_pay(c, (long long)X * N, o, N)) return 0;
-  return std::max(dgemm_tc_workspace(X * N, o, N), dgemm_tc_workspace(X * o, N - o, N));
-}
-
+// biq[Q][i][nu] (transform_ri, ri.cc:147-172), on the FP64 pipe, and on the digit
+// GEMM (precision forms; b[Q] symmetric, so its rows serve as its columns).
 int mo_block_fp64(corr_context* c, int X, int N, int o, const double* mos, const double* b,
                   double* biq, double* out) {
   const int v = N - o;
@@ -90,11 +80,11 @@ int mo_block_fp64(corr_context* c, int X, int N, int o, const double* mos, const
 }
 
 int mo_block_digits(corr_context* c, int X, int N, int o, const double* mos, const double* b,
-                    bool symmetric, double* biq, double* out, void* dws) {
+                    double* biq, double* out, void* dws) {
   const int v = N - o;
   // (Q|i nu): rows (Q, nu) against the occupied rows of C, written [Q][i][nu]
   DgemmTc g1;
-  g1.A = symmetric ? mat_view(b, N, 1) : MatView{b, (long long)N * N, 1, N, N};
+  g1.A = mat_view(b, N, 1);
   g1.B = mat_view(mos, N, 1);
   g1.C = OutView{biq, (long long)o * N, 1, N, N};
   g1.M = X * N;
@@ -125,13 +115,6 @@ int check_packed(int nroe, int N, long long nint, const double* mos, const long 
   return CORR_OK;
 }
 
-bool packed_overlap(const void* out, size_t bytes, int N, const void* mos, long long nint,
-                    const void* val, const void* num) {
-  return overlaps(out, bytes, mos, (size_t)N * N * 8) ||
-         (nint > 0 && (overlaps(out, bytes, val, (size_t)nint * 8) ||
-                       overlaps(out, bytes, num, (size_t)nint * 8)));
-}
-
 }  // namespace
 }  // namespace corr
 
@@ -144,35 +127,30 @@ int corr_build_fmo(corr_context* c, int nroao, const double* mos, const double* 
   CORR_CHECK_ARG(c && mos && fmat && fmo, "corr_build_fmo: null argument");
   CORR_CHECK_ARG(nroao >= 1, "corr_build_fmo: nroao must be positive");
   CORR_CUDA(cudaSetDevice(c->device));
-  const bool fp64_only = overlaps(fmo, (size_t)nroao * nroao * 8, fmat, (size_t)nroao * nroao * 8) ||
-                         overlaps(fmo, (size_t)nroao * nroao * 8, mos, (size_t)nroao * nroao * 8);
-  return with_fp64_retry(c, fp64_only, [&]() -> int {
-    const int N = nroao;
-    const size_t n2 = (size_t)N * N;
-    const bool odev = is_device_ptr(fmo);
-    Carver cv{nullptr, 0};
-    for (int k = 0; k < 4; ++k) cv.take(n2 * 8);
-    cv.take(gemm_plain_workspace(c, N, N, N));
-    CORR_TRY(c->ws.reserve(cv.used));
-    Carver w{c->ws.ptr, 0};
-    void* s_m = w.take(n2 * 8);
-    void* s_f = w.take(n2 * 8);
-    double* T = static_cast<double*>(w.take(n2 * 8));
-    double* out = odev ? fmo : static_cast<double*>(w.take(n2 * 8));
-    void* dws = w.take(gemm_plain_workspace(c, N, N, N));
-    CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
-    mark(c, 0);
-    const double* d_m = static_cast<const double*>(stage_in(c, mos, n2 * 8, s_m));
-    const double* d_f = static_cast<const double*>(stage_in(c, fmat, n2 * 8, s_f));
-    CORR_CHECK_ARG(d_m && d_f, "corr_build_fmo: host-to-device copy failed");
-    mark(c, 1);
-    // T = C F ; FMo = T C^T   (FMo[i][j] = sum C[i][mu] F[mu][nu] C[j][nu])
-    CORR_TRY(gemm_plain(c, gemm_args(d_m, d_f, T, N, N, N, N, N, N, 0, 0), dws));
-    CORR_TRY(gemm_plain(c, gemm_args(T, d_m, out, N, N, N, N, N, N, 0, 1), dws));
-    mark(c, 2);
-    CORR_TRY(stage_out(c, fmo, out, n2 * 8));
-    return finish_results(c, 0);
-  });
+  const int N = nroao;
+  const size_t n2 = (size_t)N * N;
+  const bool odev = is_device_ptr(fmo);
+  Carver cv{nullptr, 0};
+  for (int k = 0; k < 4; ++k) cv.take(n2 * 8);
+  CORR_TRY(c->ws.reserve(cv.used));
+  Carver w{c->ws.ptr, 0};
+  void* s_m = w.take(n2 * 8);
+  void* s_f = w.take(n2 * 8);
+  double* T = static_cast<double*>(w.take(n2 * 8));
+  double* out = odev ? fmo : static_cast<double*>(w.take(n2 * 8));
+  CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
+  mark(c, 0);
+  const double* d_m = static_cast<const double*>(stage_in(c, mos, n2 * 8, s_m));
+  const double* d_f = static_cast<const double*>(stage_in(c, fmat, n2 * 8, s_f));
+  CORR_CHECK_ARG(d_m && d_f, "corr_build_fmo: host-to-device copy failed");
+  mark(c, 1);
+  // T = C F ; FMo = T C^T   (FMo[i][j] = sum C[i][mu] F[mu][nu] C[j][nu])
+  CORR_TRY(gemm_f64(gemm_args(d_m, d_f, T, N, N, N, N, N, N, 0, 0), &c->dres->status, c->stream));
+  CORR_TRY(gemm_f64(gemm_args(T, d_m, out, N, N, N, N, N, N, 0, 1), &c->dres->status, c->stream));
+  c->launches += 2;
+  mark(c, 2);
+  CORR_TRY(stage_out(c, fmo, out, n2 * 8));
+  return finish_results(c, 0);
 }
 
 int corr_motrans(corr_context* c, int nroe, int nroao, const double* mos, long long nrofint,
@@ -181,36 +159,31 @@ int corr_motrans(corr_context* c, int nroe, int nroao, const double* mos, long l
   CORR_CHECK_ARG(c && prec, "corr_motrans: null argument");
   CORR_TRY(check_packed(nroe, nroao, nrofint, mos, sortcount, intval, intnums));
   CORR_CUDA(cudaSetDevice(c->device));
-  const bool fp64_only = packed_overlap(prec, (size_t)nroao * nroao * nroao * nroao * 8, nroao, mos, nrofint,
-                                        intval, intnums);
-  return with_fp64_retry(c, fp64_only, [&]() -> int {
-    const int N = nroao;
-    const size_t n4 = (size_t)N * N * N * N;
-    const bool odev = is_device_ptr(prec);
-    auto plan = [&](Carver& w, double** out) {
-      w.take((size_t)N * N * 8);
-      w.take(32);
-      w.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
-      w.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
-      w.take(n4 * 8);
-      w.take(n4 * 8);
-      w.take(quarter_workspace(c, N));
-      *out = odev ? prec : static_cast<double*>(w.take(n4 * 8));
-    };
-    double* out;
-    Carver cv{nullptr, 0};
-    plan(cv, &out);
-    CORR_TRY(c->ws.reserve(cv.used));
-    CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
-    mark(c, 0);
-    Carver w{c->ws.ptr, 0};
-    // the same carving order as plan(): staging buffers first, output last
-    Carver w2 = w;
-    plan(w2, &out);
-    CORR_TRY(motrans_device(c, w, nroe, N, mos, nrofint, sortcount, intval, intnums, true, out));
-    CORR_TRY(stage_out(c, prec, out, n4 * 8));
-    return finish_results(c, 0);
-  });
+  const int N = nroao;
+  const size_t n4 = (size_t)N * N * N * N;
+  const bool odev = is_device_ptr(prec);
+  auto plan = [&](Carver& w, double** out) {
+    w.take((size_t)N * N * 8);
+    w.take(32);
+    w.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
+    w.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
+    w.take(n4 * 8);
+    w.take(n4 * 8);
+    *out = odev ? prec : static_cast<double*>(w.take(n4 * 8));
+  };
+  double* out;
+  Carver cv{nullptr, 0};
+  plan(cv, &out);
+  CORR_TRY(c->ws.reserve(cv.used));
+  CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
+  mark(c, 0);
+  Carver w{c->ws.ptr, 0};
+  // the same carving order as plan(): staging buffers first, output last
+  Carver w2 = w;
+  plan(w2, &out);
+  CORR_TRY(motrans_device(c, w, nroe, N, mos, nrofint, sortcount, intval, intnums, true, out));
+  CORR_TRY(stage_out(c, prec, out, n4 * 8));
+  return finish_results(c, 0);
 }
 
 int corr_motrans_ovov(corr_context* c, int nroe, int nroao, const double* mos, long long nrofint,
@@ -219,43 +192,36 @@ int corr_motrans_ovov(corr_context* c, int nroe, int nroao, const double* mos, l
   CORR_CHECK_ARG(c && ovov, "corr_motrans_ovov: null argument");
   CORR_TRY(check_packed(nroe, nroao, nrofint, mos, sortcount, intval, intnums));
   CORR_CUDA(cudaSetDevice(c->device));
-  const bool fp64_only = packed_overlap(
-      ovov, (size_t)(nroe / 2) * (nroao - nroe / 2) * (nroe / 2) * (nroao - nroe / 2) * 8, nroao, mos,
-      nrofint, intval, intnums);
-  return with_fp64_retry(c, fp64_only, [&]() -> int {
-    const int N = nroao, o = nroe / 2, v = N - o;
-    const size_t n4 = (size_t)N * N * N * N, nov = (size_t)o * v * o * v;
-    const bool odev = is_device_ptr(ovov);
-    Carver cv{nullptr, 0};
-    cv.take((size_t)N * N * 8);
-    cv.take(32);
-    cv.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
-    cv.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
-    cv.take(n4 * 8);
-    cv.take(n4 * 8);
-    cv.take(quarter_workspace(c, N));
-    if (!odev) cv.take(nov * 8);
-    CORR_TRY(c->ws.reserve(cv.used));
-    CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
-    mark(c, 0);
-    Carver w{c->ws.ptr, 0};
-    Carver wo = w;
-    double* out = ovov;
-    if (!odev) {
-      // output staging lives after the motrans buffers
-      wo.take((size_t)N * N * 8);
-      wo.take(32);
-      wo.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
-      wo.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
-      wo.take(n4 * 8);
-      wo.take(n4 * 8);
-      wo.take(quarter_workspace(c, N));
-      out = static_cast<double*>(wo.take(nov * 8));
-    }
-    CORR_TRY(motrans_device(c, w, nroe, N, mos, nrofint, sortcount, intval, intnums, false, out));
-    CORR_TRY(stage_out(c, ovov, out, nov * 8));
-    return finish_results(c, 0);
-  });
+  const int N = nroao, o = nroe / 2, v = N - o;
+  const size_t n4 = (size_t)N * N * N * N, nov = (size_t)o * v * o * v;
+  const bool odev = is_device_ptr(ovov);
+  Carver cv{nullptr, 0};
+  cv.take((size_t)N * N * 8);
+  cv.take(32);
+  cv.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
+  cv.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
+  cv.take(n4 * 8);
+  cv.take(n4 * 8);
+  if (!odev) cv.take(nov * 8);
+  CORR_TRY(c->ws.reserve(cv.used));
+  CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
+  mark(c, 0);
+  Carver w{c->ws.ptr, 0};
+  Carver wo = w;
+  double* out = ovov;
+  if (!odev) {
+    // output staging lives after the motrans buffers
+    wo.take((size_t)N * N * 8);
+    wo.take(32);
+    wo.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
+    wo.take((size_t)(nrofint > 0 ? nrofint : 1) * 8);
+    wo.take(n4 * 8);
+    wo.take(n4 * 8);
+    out = static_cast<double*>(wo.take(nov * 8));
+  }
+  CORR_TRY(motrans_device(c, w, nroe, N, mos, nrofint, sortcount, intval, intnums, false, out));
+  CORR_TRY(stage_out(c, ovov, out, nov * 8));
+  return finish_results(c, 0);
 }
 
 static int canonical_common(corr_context* c, const double* t, int full, int N, int o, int v,
@@ -311,42 +277,30 @@ int corr_transform_ri(corr_context* c, int nroe, int nroao, int naux, const doub
                  "corr_transform_ri: need naux >= 1 and even nroe with 0 < nroe/2 < nroao");
   CORR_CHECK_ARG(naux <= 65535, "corr_transform_ri: naux > 65535");
   CORR_CUDA(cudaSetDevice(c->device));
-  const bool fp64_only = overlaps(bia, (size_t)naux * (nroe / 2) * (nroao - nroe / 2) * 8, bpq,
-                                  (size_t)naux * nroao * nroao * 8) ||
-                         overlaps(bia, (size_t)naux * (nroe / 2) * (nroao - nroe / 2) * 8, mos,
-                                  (size_t)nroao * nroao * 8);
-  return with_fp64_retry(c, fp64_only, [&]() -> int {
-    const int N = nroao, o = nroe / 2, v = N - o, X = naux;
-    const size_t nb = (size_t)X * N * N, nbia = (size_t)X * o * v, nbiq = (size_t)X * o * N;
-    const bool mdev = is_device_ptr(mos), bdev = is_device_ptr(bpq), odev = is_device_ptr(bia);
-    Carver cv{nullptr, 0};
-    if (!mdev) cv.take((size_t)N * N * 8);
-    if (!bdev) cv.take(nb * 8);
-    cv.take(nbiq * 8);
-    if (!odev) cv.take(nbia * 8);
-    const size_t dws_bytes = mo_block_workspace(c, X, N, o);
-    cv.take(dws_bytes);
-    CORR_TRY(c->ws.reserve(cv.used));
-    Carver w{c->ws.ptr, 0};
-    void* s_m = mdev ? nullptr : w.take((size_t)N * N * 8);
-    void* s_b = bdev ? nullptr : w.take(nb * 8);
-    double* biq = static_cast<double*>(w.take(nbiq * 8));
-    double* out = odev ? bia : static_cast<double*>(w.take(nbia * 8));
-    void* dws = w.take(dws_bytes);
-    CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
-    mark(c, 0);
-    const double* d_m = static_cast<const double*>(stage_in(c, mos, (size_t)N * N * 8, s_m));
-    const double* d_b = static_cast<const double*>(stage_in(c, bpq, nb * 8, s_b));
-    CORR_CHECK_ARG(d_m && d_b, "host-to-device copy failed");
-    mark(c, 1);
-    if (dws_bytes)
-      CORR_TRY(mo_block_digits(c, X, N, o, d_m, d_b, false, biq, out, dws));
-    else
-      CORR_TRY(mo_block_fp64(c, X, N, o, d_m, d_b, biq, out));
-    mark(c, 2);
-    CORR_TRY(stage_out(c, bia, out, nbia * 8));
-    return finish_results(c, 0);
-  });
+  const int N = nroao, o = nroe / 2, v = N - o, X = naux;
+  const size_t nb = (size_t)X * N * N, nbia = (size_t)X * o * v, nbiq = (size_t)X * o * N;
+  const bool mdev = is_device_ptr(mos), bdev = is_device_ptr(bpq), odev = is_device_ptr(bia);
+  Carver cv{nullptr, 0};
+  if (!mdev) cv.take((size_t)N * N * 8);
+  if (!bdev) cv.take(nb * 8);
+  cv.take(nbiq * 8);
+  if (!odev) cv.take(nbia * 8);
+  CORR_TRY(c->ws.reserve(cv.used));
+  Carver w{c->ws.ptr, 0};
+  void* s_m = mdev ? nullptr : w.take((size_t)N * N * 8);
+  void* s_b = bdev ? nullptr : w.take(nb * 8);
+  double* biq = static_cast<double*>(w.take(nbiq * 8));
+  double* out = odev ? bia : static_cast<double*>(w.take(nbia * 8));
+  CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
+  mark(c, 0);
+  const double* d_m = static_cast<const double*>(stage_in(c, mos, (size_t)N * N * 8, s_m));
+  const double* d_b = static_cast<const double*>(stage_in(c, bpq, nb * 8, s_b));
+  CORR_CHECK_ARG(d_m && d_b, "host-to-device copy failed");
+  mark(c, 1);
+  CORR_TRY(mo_block_fp64(c, X, N, o, d_m, d_b, biq, out));
+  mark(c, 2);
+  CORR_TRY(stage_out(c, bia, out, nbia * 8));
+  return finish_results(c, 0);
 }
 
 int corr_ri_build_bpq(corr_context* c, int naux, int nroao, const double* jm12,
@@ -354,35 +308,32 @@ int corr_ri_build_bpq(corr_context* c, int naux, int nroao, const double* jm12,
   CORR_CHECK_ARG(c && jm12 && pmn && bpq, "corr_ri_build_bpq: null argument");
   CORR_CHECK_ARG(naux >= 1 && nroao >= 1, "corr_ri_build_bpq: sizes must be positive");
   CORR_CUDA(cudaSetDevice(c->device));
-  const bool fp64_only = false;
-  return with_fp64_retry(c, fp64_only, [&]() -> int {
-    const int X = naux;
-    const long long N2 = (long long)nroao * nroao;
-    CORR_CHECK_ARG(N2 <= 0x7fffffffLL, "corr_ri_build_bpq: nroao^2 too large");
-    const size_t np = (size_t)X * N2, nj = (size_t)X * X;
-    const bool jdev = is_device_ptr(jm12), pdev = is_device_ptr(pmn), odev = is_device_ptr(bpq);
-    Carver cv{nullptr, 0};
-    if (!jdev) cv.take(nj * 8);
-    if (!pdev) cv.take(np * 8);
-    if (!odev) cv.take(np * 8);
-    cv.take(gemm_plain_workspace(c, X, N2, X));
-    CORR_TRY(c->ws.reserve(cv.used));
-    Carver w{c->ws.ptr, 0};
-    void* s_j = jdev ? nullptr : w.take(nj * 8);
-    void* s_p = pdev ? nullptr : w.take(np * 8);
-    double* out = odev ? bpq : static_cast<double*>(w.take(np * 8));
-    void* dws = w.take(gemm_plain_workspace(c, X, N2, X));
-    CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
-    mark(c, 0);
-    const double* d_j = static_cast<const double*>(stage_in(c, jm12, nj * 8, s_j));
-    const double* d_p = static_cast<const double*>(stage_in(c, pmn, np * 8, s_p));
-    CORR_CHECK_ARG(d_j && d_p, "host-to-device copy failed");
-    mark(c, 1);
-    CORR_TRY(gemm_plain(c, gemm_args(d_j, d_p, out, X, (int)N2, X, X, N2, N2, 0, 0), dws));
-    mark(c, 2);
-    CORR_TRY(stage_out(c, bpq, out, np * 8));
-    return finish_results(c, 0);
-  });
+  const int X = naux;
+  const long long N2 = (long long)nroao * nroao;
+  CORR_CHECK_ARG(N2 <= 0x7fffffffLL, "corr_ri_build_bpq: nroao^2 too large");
+  const size_t np = (size_t)X * N2, nj = (size_t)X * X;
+  const bool jdev = is_device_ptr(jm12), pdev = is_device_ptr(pmn), odev = is_device_ptr(bpq);
+  Carver cv{nullptr, 0};
+  if (!jdev) cv.take(nj * 8);
+  if (!pdev) cv.take(np * 8);
+  if (!odev) cv.take(np * 8);
+  CORR_TRY(c->ws.reserve(cv.used));
+  Carver w{c->ws.ptr, 0};
+  void* s_j = jdev ? nullptr : w.take(nj * 8);
+  void* s_p = pdev ? nullptr : w.take(np * 8);
+  double* out = odev ? bpq : static_cast<double*>(w.take(np * 8));
+  CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
+  mark(c, 0);
+  const double* d_j = static_cast<const double*>(stage_in(c, jm12, nj * 8, s_j));
+  const double* d_p = static_cast<const double*>(stage_in(c, pmn, np * 8, s_p));
+  CORR_CHECK_ARG(d_j && d_p, "host-to-device copy failed");
+  mark(c, 1);
+  CORR_TRY(gemm_f64(gemm_args(d_j, d_p, out, X, (int)N2, X, X, N2, N2, 0, 0), &c->dres->status,
+                    c->stream));
+  c->launches += 1;
+  mark(c, 2);
+  CORR_TRY(stage_out(c, bpq, out, np * 8));
+  return finish_results(c, 0);
 }
 
 }  // extern "C"
@@ -535,33 +486,29 @@ int corr_ri_apply_metric(corr_context* c, int naux, long long ncols, const doubl
   CORR_CHECK_ARG(naux >= 1 && ncols >= 1 && ncols <= 0x7fffffffLL,
                  "corr_ri_apply_metric: bad sizes");
   CORR_CUDA(cudaSetDevice(c->device));
-  const bool fp64_only = false;
-  return with_fp64_retry(c, fp64_only, [&]() -> int {
-    const size_t nj = (size_t)naux * naux, nx = (size_t)naux * ncols;
-    const bool jdev = is_device_ptr(jm12), idev = is_device_ptr(in), odev = is_device_ptr(out);
-    Carver cv{nullptr, 0};
-    if (!jdev) cv.take(nj * 8);
-    if (!idev) cv.take(nx * 8);
-    if (!odev) cv.take(nx * 8);
-    cv.take(gemm_plain_workspace(c, naux, ncols, naux));
-    CORR_TRY(c->ws.reserve(cv.used));
-    Carver w{c->ws.ptr, 0};
-    void* s_j = jdev ? nullptr : w.take(nj * 8);
-    void* s_i = idev ? nullptr : w.take(nx * 8);
-    double* o = odev ? out : static_cast<double*>(w.take(nx * 8));
-    void* dws = w.take(gemm_plain_workspace(c, naux, ncols, naux));
-    CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
-    mark(c, 0);
-    const double* d_j = static_cast<const double*>(stage_in(c, jm12, nj * 8, s_j));
-    const double* d_i = static_cast<const double*>(stage_in(c, in, nx * 8, s_i));
-    CORR_CHECK_ARG(d_j && d_i, "host-to-device copy failed");
-    mark(c, 1);
-    CORR_TRY(gemm_plain(
-        c, gemm_args(d_j, d_i, o, naux, (int)ncols, naux, naux, ncols, ncols, 0, 0), dws));
-    mark(c, 2);
-    CORR_TRY(stage_out(c, out, o, nx * 8));
-    return finish_results(c, 0);
-  });
+  const size_t nj = (size_t)naux * naux, nx = (size_t)naux * ncols;
+  const bool jdev = is_device_ptr(jm12), idev = is_device_ptr(in), odev = is_device_ptr(out);
+  Carver cv{nullptr, 0};
+  if (!jdev) cv.take(nj * 8);
+  if (!idev) cv.take(nx * 8);
+  if (!odev) cv.take(nx * 8);
+  CORR_TRY(c->ws.reserve(cv.used));
+  Carver w{c->ws.ptr, 0};
+  void* s_j = jdev ? nullptr : w.take(nj * 8);
+  void* s_i = idev ? nullptr : w.take(nx * 8);
+  double* o = odev ? out : static_cast<double*>(w.take(nx * 8));
+  CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
+  mark(c, 0);
+  const double* d_j = static_cast<const double*>(stage_in(c, jm12, nj * 8, s_j));
+  const double* d_i = static_cast<const double*>(stage_in(c, in, nx * 8, s_i));
+  CORR_CHECK_ARG(d_j && d_i, "host-to-device copy failed");
+  mark(c, 1);
+  CORR_TRY(gemm_f64(gemm_args(d_j, d_i, o, naux, (int)ncols, naux, naux, ncols, ncols, 0, 0),
+                    &c->dres->status, c->stream));
+  c->launches += 1;
+  mark(c, 2);
+  CORR_TRY(stage_out(c, out, o, nx * 8));
+  return finish_results(c, 0);
 }
 
 int corr_rimp2_energy_from_3index(corr_context* c, int nroe, int nroao, int naux,
@@ -581,11 +528,12 @@ int corr_rimp2_energy_from_3index(corr_context* c, int nroe, int nroao, int naux
                  nj = (size_t)X * X;
     const bool mdev = is_device_ptr(mos), edev = is_device_ptr(eps), jdev = is_device_ptr(J),
                pdev = is_device_ptr(pmn);
-    // The FP64 contractions run on the tensor cores (dgemm_tc.cu, FP64-accurate
-    // digit slicing); the plain form of a strict context and small plain problems
-    // keep the FP64 pipe throughout.
-    const bool tc = precision != CORR_PREC_FP64 ||
-                  digits_pay(c, (long long)naux * nroao, nroe / 2, nroao);
+    // The precision forms run the FP64 contractions on the tensor cores
+    // (dgemm_tc.cu, FP64-accurate digit slicing).  The plain form keeps them on the
+    // FP64 pipe: with a wide range inside the rows (C and L^-1 of a real metric)
+    // the digit GEMM's normwise error is 3 to 6 times the FP64 GEMM's there; only
+    // the (ia|jb) panels of its energy, where it is smaller, use the digits.
+    const bool tc = precision != CORR_PREC_FP64;
     const bool panels = energy_on_panels(c, nroe / 2, nroao - nroe / 2, naux, precision);
     // Region 1 (persistent across the stages): staged inputs, (P|ia), B, J^-1/2.
     auto plan = [&](Carver& w, void** sm, void** se, void** sj, void** sp, double** pia,
@@ -646,7 +594,7 @@ int corr_rimp2_energy_from_3index(corr_context* c, int nroe, int nroao, int naux
       // cluster, whole pipeline: 16.3 ms with none left, 15.7 with 2, 14.8 with
       // 12, 14.4 with 24, 14.7 with 40.
       c->spare_sms = 24;
-      const int st = mo_block_digits(c, X, N, o, d_m, d_p, true, biq, pia, dws);
+      const int st = mo_block_digits(c, X, N, o, d_m, d_p, biq, pia, dws);
       c->spare_sms = 0;
       CORR_TRY(st);
       {

@@ -17,7 +17,6 @@
 // of the hot path: build_FMo, the four MOtrans quarter transforms, transform_ri,
 // the RI B build and the J^-1/2 assembly.
 #include "common.cuh"
-#include "dgemm_tc.h"
 #include "gemm_fp64.h"
 
 namespace corr {
@@ -283,12 +282,13 @@ bool aligned16(const void* p, long long ld) {
 
 int gemm_f64(const GemmF64& g, int* status, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return CORR_OK;
-  // small tiles where they leave the busiest SM less than half of the 64 x 64
-  // tiles' work (their loads go through registers, so a smaller margin is not
-  // worth taking); 8 x 8 where they save another sixth
+  // small tiles where they save the busiest SM a fifth of the 64 x 64 tiles' work
+  // (they reach 0.8 to 0.9 of the FP64 pipe's rate); 8 x 8 where they save another
+  // sixth.  (A transform of 43 occupied rows over 227 functions, for instance, pads
+  // to 64 x 256 in 64 x 64 tiles.)
   const double w64 = busiest_sm(g, BM, BK), w16 = busiest_sm(g, 16, 1), w8 = busiest_sm(g, 8, 1);
   const bool fits = g.batch <= 65535 && (g.N + 7) / 8 <= 65535;
-  if (fits && 2.0 * w16 <= w64) return 1.2 * w8 <= w16 ? launch_small<8>(g, s) : launch_small<16>(g, s);
+  if (fits && 1.25 * w16 <= w64) return 1.2 * w8 <= w16 ? launch_small<8>(g, s) : launch_small<16>(g, s);
   CUtensorMap ta{}, tb{};
   // TMA needs 16-byte aligned base/leading dimension and batch strides
   bool tmaA = aligned16(g.A, g.lda) && (g.sa * 8) % 16 == 0 && g.K > 0;
@@ -327,28 +327,6 @@ int gemm_f64(const GemmF64& g, int* status, cudaStream_t s) {
     return CORR_ERR_CUDA;
   }
   return CORR_OK;
-}
-
-size_t gemm_plain_workspace(const corr_context* c, long long M, long long N, long long K) {
-  return digits_pay(c, M, N, K) ? dgemm_tc_workspace((int)M, (int)N, (int)K) : 0;
-}
-
-int gemm_plain(corr_context* c, const GemmF64& g, void* ws) {
-  if (!digits_pay(c, g.M, g.N, g.K) || g.batch != 1 || g.beta != 0.0) {
-    c->launches += 1;
-    return gemm_f64(g, &c->dres->status, c->stream);
-  }
-  DgemmTc d;
-  d.A = g.ta ? mat_view(g.A, 1, g.lda) : mat_view(g.A, g.lda, 1);
-  d.B = g.tb ? mat_view(g.B, g.ldb, 1) : mat_view(g.B, 1, g.ldb);
-  d.C = out_view(g.C, g.ldc, 1);
-  d.M = g.M;
-  d.N = g.N;
-  d.K = g.K;
-  d.alpha = g.alpha;
-  d.accumulate = false;
-  d.a_lower = false;
-  return dgemm_tc(c, d, ws);
 }
 
 }  // namespace corr

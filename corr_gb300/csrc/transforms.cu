@@ -116,13 +116,13 @@ int grid_for(long long n, int sms) {
 // One quarter transform: out[r][p] = sum_a in[a][r] C[p][a] for the nout rows
 // of C starting at `crow` (in: K x M with K = N).
 int quarter(corr_context* c, const double* in, const double* mos, int N, int crow, int nout,
-            long long M, double* out, void* dws) {
+            long long M, double* out) {
   if (M > 0x7fffffffLL) {
     set_error("quarter transform: %lld rows exceed the GEMM row limit", M);
     return CORR_ERR_BAD_ARG;
   }
   GemmF64 g = gemm_args(in, mos + (size_t)crow * N, out, (int)M, nout, N, M, N, nout, 1, 1);
-  return gemm_plain(c, g, dws);
+  return gemm_f64(g, &c->dres->status, c->stream);
 }
 
 int launch_unpack(corr_context* c, int N, long long n, const long long* sc, const double* val,

@@ -45,11 +45,11 @@ enum corr_status {
 
 /* Arithmetic of the RI-MP2 contraction (ia|jb) = sum_Q B^Q_ia B^Q_jb. */
 enum corr_precision {
-  CORR_PREC_FP64 = 0,       /* the plain form: FP64 accuracy end to end.  Large
-                               products run on the FP64-accurate digit GEMM
-                               (corr_dgemm_tc), everything else and the products
-                               of a strict context (corr_set_fp64_strict) on the
-                               FP64 pipe                                         */
+  CORR_PREC_FP64 = 0,       /* the plain form: FP64 end to end on the FP64 pipe;
+                               the (ia|jb) panels of large energies and the
+                               gradient's products on the FP64-accurate digit
+                               GEMM (corr_dgemm_tc) unless the context is strict
+                               (corr_set_fp64_strict)                            */
   CORR_PREC_SPLIT_FP16 = 1, /* each row (i,a) of B scaled by a power of two and
                                split into two integer digits s0 + s1/L stored as
                                FP16 (|digit| <= 2048); the products s0.s0',
@@ -187,18 +187,17 @@ int corr_selftest_wait_timeout(corr_context* ctx, int limit_ms);
 int corr_set_energy_tiles(corr_context* ctx, int tiles);
 
 /* FP64 arithmetic of the plain form (no counterpart in the reference).  0 (the
- * default): the large products of the plain-form calls (corr_rimp2_energy and
- * corr_rimp2_energy_from_3index with CORR_PREC_FP64, corr_rimp2_gradient,
- * corr_transform_ri, corr_build_fmo, corr_motrans, corr_ri_build_bpq,
- * corr_ri_apply_metric, corr_calculate_ri) run on the FP64-accurate digit GEMM
- * (corr_dgemm_tc), and J^-1/2 of a certified metric is computed by
- * Newton-Schulz on it (5e-11 from LAPACK's on the 20-water cluster); inputs
- * outside the digit GEMM's range (not finite, rows of subnormals) repeat the
- * call on the FP64 pipe (corr_calculate_ri expects finite inputs).  1: every
- * product on the FP64 pipe and J^-1/2 by the
- * eigendecomposition -- IEEE FP64 end to end, many times slower.
- * corr_rimp2_energy_async, the batched calls and corr_rimp2_energy_noalloc run
- * their FP64 form on the FP64 pipe in either mode. */
+ * default): the (ia|jb) panels of corr_rimp2_energy and
+ * corr_rimp2_energy_from_3index with CORR_PREC_FP64, the products of
+ * corr_rimp2_gradient and of corr_calculate_ri run on the FP64-accurate digit
+ * GEMM (corr_dgemm_tc), and J^-1/2 of a certified metric is computed by
+ * Newton-Schulz on it (5e-11 from LAPACK's on the 20-water cluster); a B outside
+ * the digit GEMM's range (not finite, rows of subnormals) repeats the energy or
+ * gradient on the FP64 pipe.  1: every product on the FP64 pipe and J^-1/2 by the
+ * eigendecomposition -- IEEE FP64 end to end, many times slower.  The transforms
+ * and corr_ri_build_bpq / corr_ri_apply_metric run on the FP64 pipe in either
+ * mode, as do the FP64 forms of corr_rimp2_energy_async, of the batched calls and
+ * of corr_rimp2_energy_noalloc. */
 int corr_set_fp64_strict(corr_context* ctx, int strict);
 
 /* Launch variant of the batched kernel: unit order (0 = input order,
@@ -257,7 +256,7 @@ int corr_rimp2_energy_noalloc(int device, void* stream, int nocc, int nvir, int 
 
 /* Replaces build_FMo (src/POSTHF/motrans.cc:8-32, declared at
  * src/POSTHF/motrans.h:22): fmo[i*N+j] = sum_{mu,nu} mos[i*N+mu] fmat[mu*N+nu]
- * mos[j*N+nu], as two FP64-accurate GEMMs.  The caller owns fmo (N*N). */
+ * mos[j*N+nu], as two FP64 GEMMs.  The caller owns fmo (N*N). */
 int corr_build_fmo(corr_context* ctx, int nroao, const double* mos, const double* fmat,
                    double* fmo);
 

@@ -1,6 +1,7 @@
-"""The plain form's routes: FP64-accurate panels and products on the digit GEMM
-(the default from a few 1e7 multiply-adds on) against the FP64 pipe
-(set_fp64_strict) and the oracle, on both sides of the rules' lines.
+"""The plain form's routes: the energy and the gradient from FP64-accurate panels on
+the digit GEMM (the default; the energy from 3e7 multiply-adds on) against the FP64
+pipe (set_fp64_strict) and the oracle, on both sides of the rule's line, and the
+transforms and metric products, which stay on the FP64 pipe.
 
 Tolerances: the repository's FP64 bounds, 1e-12 relative for energies and 1e-11
 of the largest component for gradients; transforms 1e-13 of the largest element
