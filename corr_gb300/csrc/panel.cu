@@ -234,6 +234,10 @@ int panel_product(corr_context* c, int o, int v, int X, const double* bia, const
 int launch_panel(corr_context* c, const PanelView& pv, const double* eps, double* deps,
                  double* part, int split, bool grad) {
   const dim3 grid((unsigned)(pv.ni * (pv.o - pv.i0)), (unsigned)split);
+  // the W sums of a long virtual range go beyond the 48 KB that need no opt-in
+  if (grad && pv.v > 4096)
+    CORR_CUDA(cudaFuncSetAttribute(panel_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   pv.v * 8));
   if (grad)
     panel_kernel<true><<<grid, 256, (size_t)pv.v * 8, c->stream>>>(pv, eps, deps, part);
   else

@@ -101,7 +101,7 @@ def test_infinities_propagate_as_on_the_fp64_pipe(ctx):
 
 
 @pytest.mark.parametrize("o,v,x", [(3, 7, 9), (9, 64, 70), (11, 65, 40), (5, 131, 2050),
-                                   (60, 200, 16)])
+                                   (60, 200, 16), (1, 5300, 5)])
 def test_gradient(ctx, o, v, x):
     B, eps = O.synth_rimp2(o, v, x, 7 * o + v + x)
     got = ctx.rimp2_gradient(B, eps, o, v, x)
