@@ -569,17 +569,16 @@ int make_basis(const corr_basis* b, const double sph[kLmax + 1][2 * kLmax + 1][1
                      b->coefs,
                  "corr_ri_integrals: bad %s basis", what);
   out->sh.resize(b->nsh);
-  int nprim_total = 0;
   for (int s = 0; s < b->nsh; ++s) {
     CORR_CHECK_ARG(b->l[s] >= 0 && b->l[s] <= kLmax,
                    "corr_ri_integrals: %s shell %d has l = %d (supported: 0..%d)", what, s,
                    b->l[s], kLmax);
     CORR_CHECK_ARG(b->nprim[s] >= 1 && b->poff[s] >= 0,
                    "corr_ri_integrals: %s shell %d: bad primitives", what, s);
-    nprim_total = std::max(nprim_total, b->poff[s] + b->nprim[s]);
   }
-  out->exps.assign(b->exps, b->exps + nprim_total);
-  out->cofs.assign(nprim_total, 0.0);
+  // Every shell gets primitives of its own: their coefficients carry its angular
+  // momentum's norm and, on the auxiliary side, the shell's, while the caller's
+  // shells may share a range or overlap in it.
   int bf = 0;
   for (int s = 0; s < b->nsh; ++s) {
     const int l = b->l[s];
@@ -589,15 +588,16 @@ int make_basis(const corr_basis* b, const double sph[kLmax + 1][2 * kLmax + 1][1
     d.z = b->center[3 * s + 2];
     d.l = l;
     d.nprim = b->nprim[s];
-    d.poff = b->poff[s];
+    d.poff = (int)out->exps.size();
     d.bf = bf;
     out->maxl = std::max(out->maxl, l);
-    for (int k = 0; k < d.nprim; ++k) {
-      const double a = b->exps[d.poff + k];
+    for (int k = b->poff[s]; k < b->poff[s] + d.nprim; ++k) {
+      const double a = b->exps[k];
       CORR_CHECK_ARG(a > 0.0, "corr_ri_integrals: %s shell %d: exponent must be positive", what, s);
       // x^l exp(-a r^2) normalised: (2a/pi)^(3/4) (4a)^(l/2) / sqrt((2l-1)!!)
-      out->cofs[d.poff + k] = b->coefs[d.poff + k] * std::pow(2.0 * a / M_PI, 0.75) *
-                              std::pow(4.0 * a, 0.5 * l) / std::sqrt(dfact(2 * l - 1));
+      out->exps.push_back(a);
+      out->cofs.push_back(b->coefs[k] * std::pow(2.0 * a / M_PI, 0.75) *
+                          std::pow(4.0 * a, 0.5 * l) / std::sqrt(dfact(2 * l - 1)));
     }
     // self-overlap of the contracted spherical functions (one centre):
     // S_ij = sum_pq c_p c_q prod_dim m(e_i + e_j, a_p + a_q),
