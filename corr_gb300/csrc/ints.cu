@@ -103,8 +103,10 @@ __device__ double d_boys_exp[kBoysPoints];     // e^-T_i
 template <int NMAX>
 __device__ __forceinline__ void boys(double T, double* F) {
   static_assert(NMAX <= kBoysMax, "Boys table orders");
-  // (compared as integers: T >= 0, and an FP64 compare is an FP64 instruction)
-  if (__double_as_longlong(T) < __double_as_longlong(kBoysTmax)) {
+  // (compared as integers: T >= 0, and an FP64 compare is an FP64 instruction;
+  // unsigned, so that a NaN of either sign stays out of the table)
+  if ((unsigned long long)__double_as_longlong(T) <
+      (unsigned long long)__double_as_longlong(kBoysTmax)) {
     // T * 16 to the nearest integer: 2^52 + 2^51 leaves it in the low word
     const double y = fma(T, (double)kBoysPerUnit, 6755399441055744.0);
     const int i = __double2loint(y);
