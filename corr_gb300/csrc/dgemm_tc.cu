@@ -4,9 +4,9 @@
 // two transform_ri products (src/POSTHF/ri.cc:147-172) and the metric
 // application B = L^-1 (P|ia) (the calculate_ri product, ri.cc:102-103).
 //
-// Slicing.  Row r of an operand is scaled by 2^-e_r (e_r: the binary exponent
-// of its largest element, so every scaled value lies in (-1, 1)) and written
-// as eight balanced base-128 digits,
+// Slicing.  Per pass of 512 of K, row r of an operand is scaled by 2^-e_r (e_r:
+// the binary exponent of its largest element there, so every scaled value lies
+// in (-1, 1)) and written as eight balanced base-128 digits,
 //   x / 2^e_r = sum_{s=0..7} d_s 2^(-7 (s+1)) + rho,  |d_0| <= 128,
 //   |d_s| <= 64 (s >= 1),  |rho| <= 2^-57,
 // computed with integer operations on the FP64 bit pattern (no FP64
@@ -20,9 +20,11 @@
 // in magnitude -- (L+1) products of at most 128 * 64 per k, or 128^2 for
 // L = 0 -- so its FP32 accumulation in TMEM is exact; levels 6 and 7 carry
 // weights 2^-56 and 2^-63 and their FP32 rounding is far below FP64 rounding.
-// Longer K runs in passes of 512 whose integer level sums add up exactly in
-// registers (one launch and one rounding per 2048 of K); chunks of 2048
-// accumulate into C.
+// Longer K runs in passes of 512, each with its own scales and one rounding,
+// that accumulate into C in FP64 (up to four passes in a launch).  One scale for
+// four passes would save that accumulation, but an element then keeps fewer
+// bits wherever its row is larger in another pass: rows that are large in
+// opposite passes (a factor 1e11) lost half of their digits.
 //
 // Tensor-core layout.  Output tile 128 x 64.  The eight digit planes of the
 // column operand are stacked along N in shared memory (plane t = rows
@@ -32,11 +34,12 @@
 // 256 columns is issued as two, reusing A through the collector buffer.
 //
 // Recombination (epilogue, per element): the exact levels 0..5 in a 64-bit
-// integer and levels 6..7 in FP32, summed over the passes; one rounding to
-// FP64, in integer instructions.  TMEM holds one set of level blocks, so the
-// MMAs wait while a pass's sums are read: that part is only conversion and
-// integer multiply-adds (about 25 instructions per element, eight warps), and
-// the normalisation, scaling and stores run under the next tile's MMAs.
+// integer and levels 6..7 in FP32; one rounding to FP64, in integer
+// instructions.  TMEM holds one set of level blocks, so the MMAs wait while a
+// pass's sums are read: that part is only conversion and integer multiply-adds
+// (about 25 instructions per element, eight warps), and the normalisation,
+// scaling, accumulation (FP64 adds, C in L2) and stores run under the MMAs of the
+// next pass or tile.
 //
 // CTA = 10 warps, persistent, one CTA per SM, output tiles assigned round
 // robin: warp 0 bulk-copies the digit planes (two stages of 96 KB: 8 row
@@ -67,6 +70,7 @@ constexpr int DKB = 32;                   // K per stage: 64-byte tile rows
 constexpr int KPASS = 512;                // K per pass (exact levels 0..5)
 constexpr int KCHUNK = 2048;              // K per launch (digit planes in the workspace)
 constexpr int PASS_KB = KPASS / DKB;
+constexpr int PASSES = KCHUNK / KPASS;    // scales per row and launch
 // Rows per launch: the row operand's digit planes stay below about 1 GiB (at
 // least 256 row tiles, so that a narrow product still fills the SMs).
 constexpr size_t kRowPlaneBytes = (size_t)1 << 30;
@@ -92,8 +96,8 @@ __device__ __forceinline__ long long view_row(const MatView& v, long long r) {
 }
 
 // ---------------------------------------------------------------- slicing
-// The largest biased exponent of each row, em[r] (0 for a row without a normal
-// value: all digits zero).  |x| < 2^(em - 1022) over the row.
+// The largest biased exponent of each row in a pass, em[pass][r] (0 for a row
+// without a normal value: all digits zero).  |x| < 2^(em - 1022) over the row.
 __device__ __forceinline__ int row_scale(int em) { return em > 0 ? em - 1022 : 0; }
 __device__ __forceinline__ int biased_exponent(double x) {
   return (__double2hiint(x) >> 20) & 0x7FF;
@@ -163,15 +167,16 @@ __device__ __forceinline__ void store_chunk(const double (&x)[8], int er, uint16
 // The arrival counters of a product whose tiles are split over K start at zero;
 // the slicing of its row operand, just ahead of it, clears them.
 __device__ __forceinline__ void clear_tickets(unsigned* zero, int n) {
+  if (blockIdx.y) return;
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x)
     zero[x] = 0u;
 }
 
 // Slicing of an operand whose k are adjacent in memory: `lpr` lanes (a power
-// of two) take one row, find its exponent and write its digit planes in one
-// launch; the second read of the row comes from L1/L2.  Bound by HBM (8 bytes
+// of two) take one row's part of one pass (blockIdx.y), find its exponent and
+// write its digit planes in one launch; the second read comes from L1/L2.  Bound by HBM (8 bytes
 // read, 16 written per element).  Tile images [rt][kb][s] of TR x 32, zero
-// beyond rows and kn.
+// beyond rows and kn; e[pass][rows_pad].
 template <int TR>
 __global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, long long r0, int rows,
                                                          int rows_pad, int k0,
@@ -181,14 +186,16 @@ __global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, long long r0
                                                          int* __restrict__ status,
                                                          unsigned* __restrict__ zero, int nzero) {
   clear_tickets(zero, nzero);
-  const int nch = nkb * (DKB / 8);
   const int lane = threadIdx.x & 31, sub = lane & (lpr - 1), per = 32 / lpr;
   const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int b0 = blockIdx.y * PASS_KB;                   // the pass's first K block,
+  const int nch = min(PASS_KB, nkb - b0) * (DKB / 8);    // its chunks of 8 k
+  kn = min(KPASS, kn - b0 * DKB);                        // and its k
   for (long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
        g * per < rows_pad; g += nwarp) {
-    const long long r = g * per + lane / lpr;
+    const long long r = g * per + lane / lpr;  // below rows_pad, a multiple of per
     const bool live = r < rows;
-    const double* p = live ? v.p + view_row(v, r0 + r) + k0 : nullptr;
+    const double* p = live ? v.p + view_row(v, r0 + r) + (k0 + b0 * DKB) : nullptr;
     int em = 0;
     uint32_t nz = 0;
     if (live)
@@ -201,14 +208,13 @@ __global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, long long r0
       em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
       nz |= __shfl_xor_sync(0xffffffffu, nz, o);
     }
-    if (r >= rows_pad) continue;
     if (sub == 0) {
-      e[r] = em;
+      e[(size_t)blockIdx.y * rows_pad + r] = em;
       if (status && row_out_of_range(em, nz)) atomicOr(status, kStatusNeedFp64);
     }
     const int er = row_scale(em);
     const int rt = (int)(r / TR), rr = (int)(r % TR);
-    uint16_t* row = out + (size_t)rt * nkb * DS * (TR * DKB);
+    uint16_t* row = out + ((size_t)rt * nkb + b0) * DS * (TR * DKB);
     const bool vec = (reinterpret_cast<uintptr_t>(p) & 15) == 0;
     for (int kc = sub; kc < nch; kc += lpr) {
       double x[8];
@@ -234,8 +240,9 @@ __global__ void __launch_bounds__(256) slice_krow_kernel(MatView v, long long r0
 // one lane per row and eight warps over the k of a block's segment (blockIdx.y),
 // combined by a maximum in shared and global memory (e zeroed before), ...
 constexpr int kExpSeg = 256;
+static_assert(KPASS % kExpSeg == 0, "a segment lies in one pass");
 __global__ void __launch_bounds__(256) col_exponent_kernel(MatView v, long long r0, int rows,
-                                                           int k0, int kn,
+                                                           int rows_pad, int k0, int kn,
                                                            int* __restrict__ e,
                                                            int* __restrict__ status) {
   __shared__ int sm[8][32];
@@ -263,7 +270,7 @@ __global__ void __launch_bounds__(256) col_exponent_kernel(MatView v, long long 
       em = max(em, sm[q][lane]);
       nz |= snz[q][lane];
     }
-    atomicMax(&e[r], em);
+    atomicMax(&e[(size_t)(kb / KPASS) * rows_pad + r], em);
     // per segment of k: a small segment of a large row also takes the FP64 pipe
     if (status && row_out_of_range(em, nz)) atomicOr(status, kStatusNeedFp64);
   }
@@ -287,7 +294,7 @@ __global__ void __launch_bounds__(256) slice_kcol_kernel(MatView v, long long r0
     const long long r = t % rows_pad;
     const int kc2 = (int)(t / rows_pad);
     const bool live = r < rows;
-    const int er = row_scale(e[r]);
+    const int er = row_scale(e[(size_t)(kc2 / (KPASS / 16)) * rows_pad + r]);
     const double* p = live ? v.p + view_row(v, r0 + r) + (long long)k0 * v.ks : nullptr;
     const int rt = (int)(r / TR), rr = (int)(r % TR);
     uint16_t* tile = out + ((size_t)rt * nkb + (kc2 >> 1)) * DS * (TR * DKB);
@@ -307,8 +314,9 @@ __global__ void __launch_bounds__(256) slice_kcol_kernel(MatView v, long long r0
 struct DgArgs {
   const uint16_t* Ad;  // row-operand digit tiles [mt][kb][s] (128 x 32)
   const uint16_t* Bd;  // column-operand digit tiles [nt][kb][s] (64 x 32)
-  const int* ea;       // row exponents (padded)
-  const int* eb;       // column exponents (padded)
+  const int* ea;       // row exponents [pass][lea]
+  const int* eb;       // column exponents [pass][leb]
+  int lea, leb;
   OutView C;
   double alpha;        // applied when `scaled`; else alpha = +-2^alpha_exp, its sign bit in `sign`
   int alpha_exp, scaled;
@@ -318,9 +326,11 @@ struct DgArgs {
   int col_major_order;  // units nt-major (shared column tile adjacent)
   int a_lower, k0, accumulate;
   int nsplit, kper;  // parts of a tile's K blocks (kper each): units are (tile, part)
-  unsigned long long* part_hi;  // nsplit > 1: [unit][warp][column][lane] sums of the parts,
-  float* part_tail;             // and per (tile, warp) the parts that have arrived
-  unsigned* ticket;
+  int nslot;         // nsplit > 1: [tile][slot][warp][column][lane] sums, slot = part + pass,
+  unsigned long long* part_hi;
+  float* part_tail;
+  unsigned* ticket;  // per (tile, pass, warp) the parts, per (tile, warp) the passes that arrived
+  int tiles;
   long long total;
 };
 
@@ -335,8 +345,9 @@ struct DgCtl {
 };
 
 // Unit u: its tile, and the part of its K blocks.
+template <bool SPLIT>
 __device__ __forceinline__ void unit_tile(const DgArgs& a, long long u, int* mt, int* nt) {
-  if (a.nsplit > 1) u /= a.nsplit;
+  if (SPLIT) u /= a.nsplit;
   if (a.col_major_order) {
     *nt = (int)(u / a.mtn);
     *mt = (int)(u % a.mtn);
@@ -346,7 +357,7 @@ __device__ __forceinline__ void unit_tile(const DgArgs& a, long long u, int* mt,
   }
 }
 
-// K blocks of this pass that tile row mt needs (lower-triangular A: k <= m).
+// K blocks of this launch that tile row mt needs (lower-triangular A: k <= m).
 __device__ __forceinline__ int unit_kblocks(const DgArgs& a, int mt) {
   if (!a.a_lower) return a.nkb;
   const int kend = a.m0 + (mt + 1) * TM - a.k0;  // local k < kend can be nonzero
@@ -354,24 +365,24 @@ __device__ __forceinline__ int unit_kblocks(const DgArgs& a, int mt) {
 }
 
 // K blocks [*kb0, *kb1) of unit u (empty past a triangular tile's last block).
+template <bool SPLIT>
 __device__ __forceinline__ void unit_range(const DgArgs& a, long long u, int mt, int* kb0,
                                            int* kb1) {
   const int n = unit_kblocks(a, mt);
-  const int part = a.nsplit > 1 ? (int)(u % a.nsplit) : 0;
-  *kb0 = part * a.kper;
-  *kb1 = min(n, *kb0 + a.kper);
+  *kb0 = SPLIT ? (int)(u % a.nsplit) * a.kper : 0;
+  *kb1 = SPLIT ? min(n, *kb0 + a.kper) : n;
 }
 
-// Accumulator of one output element over the K passes of a tile: levels 0..5
-// as an exact 64-bit integer in level-5 units (2^-49 of the row and column
-// scales; |sum| <= 2^60 for K <= KCHUNK) and levels 6..7 in FP32 level-5 units.
+// Sums of one output element over a pass: levels 0..5 as an exact 64-bit integer
+// in level-5 units (2^-49 of the row and column scales; |sum| <= 2^58) and levels
+// 6..7 in FP32 level-5 units.
 struct ElemSum {
   unsigned long long hi;
   float tail;
 };
 // Bits of 2^23 + 2^22 (FP32): adding it to an integer |x| <= 2^22 leaves x in
 // the low bits (a conversion on the FP32 pipe; F2I runs at a quarter rate or
-// less), and the constant comes off once per tile.
+// less); the constants come off together.
 constexpr uint32_t kMagicBits = 0x4B400000u;
 constexpr float kMagic = 12582912.0f;
 constexpr unsigned long long kMagicSum =
@@ -379,29 +390,28 @@ constexpr unsigned long long kMagicSum =
     (1ull + (1ull << 7) + (1ull << 14) + (1ull << 21) + (1ull << 28) + (1ull << 35));
 
 template <bool WIDE>
-__device__ __forceinline__ void add_levels(ElemSum& a, const float (&x)[DS]) {
+__device__ __forceinline__ ElemSum combine_levels(const float (&x)[DS]) {
   int u[6];
 #pragma unroll
   for (int L = 0; L < 6; ++L)
     u[L] = WIDE ? __float2int_rn(x[L]) + (int)kMagicBits : __float_as_int(x[L] + kMagic);
-  unsigned long long v = a.hi + (unsigned long long)(long long)u[5];
+  unsigned long long v = (unsigned long long)(long long)u[5] - kMagicSum;
   v += (unsigned long long)((long long)u[4] * (1 << 7));
   v += (unsigned long long)((long long)u[3] * (1 << 14));
   v += (unsigned long long)((long long)u[2] * (1 << 21));
   v += (unsigned long long)((long long)u[1] * (1 << 28));
   v += (unsigned long long)(uint32_t)(u[0] << 3) << 32;  // u0 2^35 modulo 2^64
-  a.hi = v;
-  a.tail = fmaf(fmaf(x[7], 0.0078125f, x[6]), 0.0078125f, a.tail);
+  return ElemSum{v, fmaf(x[7], 0.0078125f, x[6]) * 0.0078125f};
 }
 
 template <bool WIDE>
-__device__ __forceinline__ void add_chunk(ElemSum* sum, const float (&lv)[DS][8]) {
+__device__ __forceinline__ void combine_chunk(ElemSum* sum, const float (&lv)[DS][8]) {
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     float x[DS];
 #pragma unroll
     for (int L = 0; L < DS; ++L) x[L] = lv[L][e];
-    add_levels<WIDE>(sum[e], x);
+    sum[e] = combine_levels<WIDE>(x);
   }
 }
 
@@ -440,6 +450,9 @@ __device__ __noinline__ double finish_slow(long long hi, float tail, int sh, uin
   return sign ? -r : r;
 }
 
+// SPLIT: tiles split over K (nsplit > 1); a kernel of its own, since its exchange
+// costs the other one registers (3 % at K above 512).
+template <bool SPLIT>
 __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -475,9 +488,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
     bool ok = true;
     for (long long u = blockIdx.x; u < a.total && ok; u += gridDim.x) {
       int mt, nt;
-      unit_tile(a, u, &mt, &nt);
+      unit_tile<SPLIT>(a, u, &mt, &nt);
       int kb0, kb1;
-      unit_range(a, u, mt, &kb0, &kb1);
+      unit_range<SPLIT>(a, u, mt, &kb0, &kb1);
       for (int kb = kb0; kb < kb1; ++kb) {
         bool got = true;
         if (lane == 0) got = mbar_wait(&ctl->empty[st], ph ^ 1, abort, status);
@@ -521,14 +534,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
       const uint64_t dbase = smem_desc(smem_u32(tiles), 16, 512, SW64);
       for (long long u = blockIdx.x; u < a.total && ok; u += gridDim.x) {
         int mt, nt;
-        unit_tile(a, u, &mt, &nt);
+        unit_tile<SPLIT>(a, u, &mt, &nt);
         int kb0, kb1;
-        unit_range(a, u, mt, &kb0, &kb1);
+        unit_range<SPLIT>(a, u, mt, &kb0, &kb1);
         if (kb1 <= kb0) continue;
         if (!mbar_wait(&ctl->aempty, (nuse & 1) ^ 1, abort, status)) break;
         tc_fence_after();
-        for (int kb = 0; kb < kb1 - kb0; ++kb) {
-          if (kb && kb % PASS_KB == 0) {  // next K pass: the epilogue takes the sums first
+        for (int kb = kb0; kb < kb1; ++kb) {
+          const bool first = kb == kb0 || kb % PASS_KB == 0;
+          if (first && kb != kb0) {  // next K pass: the epilogue takes the sums first
             tc_commit(&ctl->afull);
             ++nuse;
             if (!mbar_wait(&ctl->aempty, (nuse & 1) ^ 1, abort, status)) {
@@ -548,7 +562,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
 #pragma unroll
             for (int s = 0; s < DS; ++s) {
               const uint64_t ar = ds + (uint64_t)((s * A_PLANE + kk * 32) >> 4);
-              const uint32_t acc = (kb % PASS_KB) | kk | s ? 1u : 0u;
+              const uint32_t acc = !first || kk || s ? 1u : 0u;
               const uint32_t d = tmem + 64u * s;
               const int nblk = DS - s;  // column planes 0 .. 7 - s
               if (nblk > 4) {
@@ -583,15 +597,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
     bool ok = true;
     for (long long u = blockIdx.x; u < a.total && ok; u += gridDim.x) {
       int mt, nt;
-      unit_tile(a, u, &mt, &nt);
+      unit_tile<SPLIT>(a, u, &mt, &nt);
       int kb0, kb1;
-      unit_range(a, u, mt, &kb0, &kb1);
+      unit_range<SPLIT>(a, u, mt, &kb0, &kb1);
       if (kb1 <= kb0) continue;
-      const int np = (kb1 - kb0 + PASS_KB - 1) / PASS_KB;
-      ElemSum sum[ECOLS];
-#pragma unroll
-      for (int e = 0; e < ECOLS; ++e) sum[e] = ElemSum{0ull, 0.f};
-      for (int p = 0; p < np; ++p, ++nuse) {
+      const int pass1 = (kb1 - 1) / PASS_KB;
+      for (int pass = kb0 / PASS_KB; pass <= pass1; ++pass, ++nuse) {
         const bool got = mbar_wait(&ctl->afull, nuse & 1, abort, status);
         if (!__all_sync(0xffffffffu, got)) {
           ok = false;
@@ -600,6 +611,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
         tc_fence_after();
         // only this part holds the MMAs of the next pass up: sums into
         // registers, then the accumulators go back
+        ElemSum sum[ECOLS];
 #pragma unroll
         for (int c = 0; c < ECOLS / 8; ++c) {
           float lv[DS][8];
@@ -614,101 +626,153 @@ __global__ void __launch_bounds__(NTHREADS, 1) dgemm_tc_kernel(DgArgs a, int* st
 #pragma unroll
             for (int L = 0; L < 6; ++L) mx = fmaxf(mx, fabsf(lv[L][e]));
           if (__any_sync(0xffffffffu, mx > 4194304.f))
-            add_chunk<true>(sum + 8 * c, lv);
+            combine_chunk<true>(sum + 8 * c, lv);
           else
-            add_chunk<false>(sum + 8 * c, lv);
+            combine_chunk<false>(sum + 8 * c, lv);
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctl->aempty);
-      }
-      if (!ok) break;
-      // the magic constants of the conversions come off once per tile
-      const unsigned long long off = kMagicSum * (unsigned long long)np;
-#pragma unroll
-      for (int e = 0; e < ECOLS; ++e) sum[e].hi -= off;
-      if (a.nsplit > 1) {
-        // A part of the tile's K: the warp leaves its sums in L2, and the warp
-        // that arrives last adds the parts up (integers exactly, the FP32 tails
-        // in part order) and stores the result.  No warp waits for another.
-        const size_t slot = ((size_t)u * EWARPS + (warp - 2)) * ECOLS * 32 + lane;
-#pragma unroll
-        for (int e = 0; e < ECOLS; ++e) {
-          __stcg(&a.part_hi[slot + 32 * e], sum[e].hi);
-          __stcg(&a.part_tail[slot + 32 * e], sum[e].tail);
-        }
-        __threadfence();
-        __syncwarp();
-        const int parts = (unit_kblocks(a, mt) + a.kper - 1) / a.kper;
-        unsigned t = 0;
-        if (lane == 0) t = atomicAdd(&a.ticket[u / a.nsplit * EWARPS + (warp - 2)], 1u);
-        if (__shfl_sync(0xffffffffu, t, 0) != (unsigned)parts - 1) continue;
-        __threadfence();
-        const size_t first =
-            ((size_t)(u / a.nsplit * a.nsplit) * EWARPS + (warp - 2)) * ECOLS * 32 + lane;
-#pragma unroll
-        for (int e = 0; e < ECOLS; ++e) sum[e] = ElemSum{0ull, 0.f};
-        for (int p = 0; p < parts; ++p) {
-          const size_t at = first + (size_t)p * EWARPS * ECOLS * 32;
+        // A part of the tile's K: the warp leaves its sums in L2, and the warp that
+        // arrives last adds the parts of the pass up (integers exactly, the FP32
+        // tails in part order) and rounds; with several passes it leaves the result
+        // in L2 again, and the last of those adds the passes up in their order.  No
+        // warp waits for another.
+        const long long tile = SPLIT ? u / a.nsplit : u;
+        auto slot = [&](int part, int ps) {
+          return ((size_t)(tile * a.nslot + part + ps) * EWARPS + (warp - 2)) * ECOLS * 32 + lane;
+        };
+        auto arrive_last = [&](long long t, int count) -> bool {
+          __threadfence();
+          __syncwarp();
+          unsigned n = 0;
+          if (lane == 0) n = atomicAdd(&a.ticket[t * EWARPS + (warp - 2)], 1u);
+          const bool last = __shfl_sync(0xffffffffu, n, 0) == (unsigned)count - 1;
+          __threadfence();
+          return last;
+        };
+        const int kblocks = SPLIT ? unit_kblocks(a, mt) : 0;
+        const int q0 = SPLIT ? pass * PASS_KB / a.kper : 0;
+        const bool apart = SPLIT && kblocks > PASS_KB;  // passes added up at the end
+        if (SPLIT) {
+          const size_t mine = slot((int)(u - tile * a.nsplit), pass);
 #pragma unroll
           for (int e = 0; e < ECOLS; ++e) {
-            sum[e].hi += __ldcg(&a.part_hi[at + 32 * e]);
-            sum[e].tail += __ldcg(&a.part_tail[at + 32 * e]);
+            __stcg(&a.part_hi[mine + 32 * e], sum[e].hi);
+            __stcg(&a.part_tail[mine + 32 * e], sum[e].tail);
+          }
+          const int parts = (min(kblocks, (pass + 1) * PASS_KB) - 1) / a.kper - q0 + 1;
+          if (!arrive_last(tile * PASSES + pass, parts)) continue;
+#pragma unroll
+          for (int e = 0; e < ECOLS; ++e) sum[e] = ElemSum{0ull, 0.f};
+          for (int q = 0; q < parts; ++q) {
+            const size_t at = slot(q0 + q, pass);
+#pragma unroll
+            for (int e = 0; e < ECOLS; ++e) {
+              sum[e].hi += __ldcg(&a.part_hi[at + 32 * e]);
+              sum[e].tail += __ldcg(&a.part_tail[at + 32 * e]);
+            }
           }
         }
-      }
-      // Normalise and store, eight columns per step: a rolled loop that moves
-      // the remaining sums down the register array (unrolled over 32 columns the
-      // code ran at the rate of its instruction fetches).
-      const long long m = a.m0 + (long long)mt * TM + arow;
-      const bool mlive = m < a.M;
-      const int n0 = nt * TN + c0;
-      const int em = (mlive ? row_scale(a.ea[m - a.m0]) : 0) + a.alpha_exp - 49;
-      const int en = row_scale(a.eb[n0 + lane]);
-      double* dst = a.C.p + (m / a.C.rdiv) * a.C.rs_hi + (m % a.C.rdiv) * a.C.rs_lo +
-                    (long long)n0 * a.C.cs;
-      const bool vec = a.C.cs == 1 && !a.accumulate && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
-#pragma unroll 1
-      for (int c = 0; c < ECOLS; c += 8) {
-        double r[8];
-        uint32_t odd = 0;
+        const long long m = a.m0 + (long long)mt * TM + arow;
+        const bool mlive = m < a.M;
+        const int n0 = nt * TN + c0;
+        double* dst = a.C.p + (m / a.C.rdiv) * a.C.rs_hi + (m % a.C.rdiv) * a.C.rs_lo +
+                      (long long)n0 * a.C.cs;
+        const bool vec = a.C.cs == 1 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+        // columns c .. c + 7 of this lane's row; all loads before the first add or store
+        auto put = [&](int c, double (&r)[8], bool accumulate) {
+          const int live = mlive ? min(8, a.N - n0 - c) : 0;
+          const bool wide = vec && live == 8;
+          double* d = dst + (long long)c * a.C.cs;
+          double2* d2 = reinterpret_cast<double2*>(d);
+          if (accumulate) {
+            double o[8];
+            if (wide) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          bool x;
-          r[e] = __longlong_as_double((long long)finish_sum(
-              (long long)sum[e].hi, sum[e].tail,
-              em + __shfl_sync(0xffffffffu, en, c + e), a.sign, &x));
-          odd |= x ? 1u << e : 0u;
-        }
-        if (__any_sync(0xffffffffu, odd != 0)) {
+              for (int e = 0; e < 4; ++e) {
+                const double2 t = d2[e];
+                o[2 * e] = t.x;
+                o[2 * e + 1] = t.y;
+              }
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) o[e] = e < live ? d[(long long)e * a.C.cs] : 0.0;
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[e] += o[e];
+          }
+          if (wide) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d2[e] = make_double2(r[2 * e], r[2 * e + 1]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (e < live) d[(long long)e * a.C.cs] = r[e];
+          }
+        };
+        // Normalise and store, eight columns per step: a rolled loop that moves
+        // the remaining sums down the register array (unrolled over 32 columns the
+        // code ran at the rate of its instruction fetches).
+        const int em = (mlive ? row_scale(a.ea[(size_t)pass * a.lea + (m - a.m0)]) : 0) +
+                       a.alpha_exp - 49;
+        const int en = row_scale(a.eb[(size_t)pass * a.leb + n0 + lane]);
+        const size_t rounded = slot(q0, pass);
+#pragma unroll 1
+        for (int c = 0; c < ECOLS; c += 8) {
+          double r[8];
+          uint32_t odd = 0;
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const int sh = em + __shfl_sync(0xffffffffu, en, c + e);
-            if (odd >> e & 1)
-              r[e] = finish_slow((long long)sum[e].hi, sum[e].tail, sh, a.sign);
+            bool x;
+            r[e] = __longlong_as_double((long long)finish_sum(
+                (long long)sum[e].hi, sum[e].tail,
+                em + __shfl_sync(0xffffffffu, en, c + e), a.sign, &x));
+            odd |= x ? 1u << e : 0u;
+          }
+          if (__any_sync(0xffffffffu, odd != 0)) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const int sh = em + __shfl_sync(0xffffffffu, en, c + e);
+              if (odd >> e & 1)
+                r[e] = finish_slow((long long)sum[e].hi, sum[e].tail, sh, a.sign);
+            }
+          }
+          if (a.scaled) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[e] *= a.alpha;
+          }
+          if (apart) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              __stcg(&a.part_hi[rounded + 32 * (c + e)],
+                     (unsigned long long)__double_as_longlong(r[e]));
+          } else {
+            put(c, r, a.accumulate || pass > 0);
+          }
+#pragma unroll
+          for (int e = 0; e + 8 < ECOLS; ++e) sum[e] = sum[e + 8];
+        }
+        if (apart) {
+          const int passes = (kblocks + PASS_KB - 1) / PASS_KB;
+          if (!arrive_last((long long)a.tiles * PASSES + tile, passes)) continue;
+#pragma unroll 1
+          for (int c = 0; c < ECOLS; c += 8) {
+            double r[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[e] = 0.0;
+#pragma unroll 2
+            for (int p = 0; p < passes; ++p) {
+              const size_t at = slot(p * PASS_KB / a.kper, p) + 32 * c;
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                r[e] += __longlong_as_double((long long)__ldcg(&a.part_hi[at + 32 * e]));
+            }
+            put(c, r, a.accumulate);
           }
         }
-        if (a.scaled) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) r[e] *= a.alpha;
-        }
-        const int live = mlive ? min(8, a.N - n0 - c) : 0;
-        double* d = dst + (long long)c * a.C.cs;
-        if (vec && live == 8) {
-#pragma unroll
-          for (int e = 0; e < 8; e += 2)
-            *reinterpret_cast<double2*>(d + e) = make_double2(r[e], r[e + 1]);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (e < live) {
-              double* x = d + (long long)e * a.C.cs;
-              *x = a.accumulate ? *x + r[e] : r[e];
-            }
-        }
-#pragma unroll
-        for (int e = 0; e + 8 < ECOLS; ++e) sum[e] = sum[e + 8];
       }
+      if (!ok) break;
     }
   }
   __syncthreads();
@@ -732,16 +796,17 @@ int slice_operand(corr_context* c, const MatView& v, long long r0, int rows, int
   if (v.ks == 1) {  // k contiguous
     int lpr = 1;
     while (lpr < 32 && lpr < nkb * (DKB / 8)) lpr *= 2;
-    const int grid = std::min(ceil_div((long long)rows_pad * lpr, 256), cap);
+    const dim3 grid((unsigned)std::min(ceil_div((long long)rows_pad * lpr, 256), cap),
+                    (unsigned)ceil_div(nkb, PASS_KB));
     slice_krow_kernel<TR><<<grid, 256, 0, c->stream>>>(v, r0, rows, rows_pad, k0, kn, nkb, lpr, e,
                                                        out, status, zero, nzero);
     CORR_CUDA(cudaGetLastError());
     c->launches += 1;
     return CORR_OK;
   }
-  CORR_CUDA(cudaMemsetAsync(e, 0, (size_t)rows_pad * 4, c->stream));
+  CORR_CUDA(cudaMemsetAsync(e, 0, (size_t)rows_pad * 4 * ceil_div(kn, KPASS), c->stream));
   const dim3 eg((unsigned)ceil_div(rows, 32), (unsigned)ceil_div(kn, kExpSeg));
-  col_exponent_kernel<<<eg, 256, 0, c->stream>>>(v, r0, rows, k0, kn, e, status);
+  col_exponent_kernel<<<eg, 256, 0, c->stream>>>(v, r0, rows, rows_pad, k0, kn, e, status);
   CORR_CUDA(cudaGetLastError());
   const int grid = std::min(ceil_div((long long)rows_pad * nkb * (DKB / 16), 256), cap);
   slice_kcol_kernel<TR><<<grid, 256, 0, c->stream>>>(v, r0, rows, rows_pad, k0, kn, nkb, e, out, zero,
@@ -760,16 +825,18 @@ int slice_operand(corr_context* c, const MatView& v, long long r0, int rows, int
 // exchange through L2.  715^3 (72 tiles): 30 us with two parts, 42 us whole.
 constexpr int kSplitSms = 152;
 constexpr int kMaxSplit = 16;
-constexpr long long kMaxSplitUnits = 2 * kSplitSms;
+constexpr long long kMaxSplitSlots = 2 * kSplitSms;
 static int k_parts(long long tiles, int nkb) {
   int best = 1;
   double cost = 0.0;
   for (int s = 1; s <= kMaxSplit && s <= nkb; ++s) {
-    if (s > 1 && tiles * s > kMaxSplitUnits) break;
+    if (s > 1 && tiles * (s + ceil_div(nkb, PASS_KB) - 1) > kMaxSplitSlots) break;
     const int kper = ceil_div(nkb, s);
+    int passes = 0;  // of the part that touches most
+    for (int b = 0; b < nkb; b += kper)
+      passes = std::max(passes, (std::min(nkb, b + kper) - 1) / PASS_KB - b / PASS_KB + 1);
     const double waves = (double)((tiles * s + kSplitSms - 1) / kSplitSms);
-    const double t = waves * (kper * 2304.0 + 3000.0 * ceil_div(kper, PASS_KB)) +
-                     (s > 1 ? 6000.0 + 600.0 * s : 0.0);
+    const double t = waves * (kper * 2304.0 + 3000.0 * passes) + (s > 1 ? 6000.0 + 600.0 * s : 0.0);
     if (s == 1 || t < 0.95 * cost) {
       cost = t;
       best = s;
@@ -779,7 +846,8 @@ static int k_parts(long long tiles, int nkb) {
 }
 // Sums and tickets of any split launch: 30 MB, part of every workspace (smaller
 // products than the one a caller sized its workspace for may split further).
-constexpr size_t kSplitBytes = (size_t)kMaxSplitUnits * TM * TN * 12 + kMaxSplitUnits * EWARPS * 4;
+constexpr size_t kSplitBytes = (size_t)kMaxSplitSlots * TM * TN * 12 +
+                               kMaxSplitSlots * (PASSES + 1) * EWARPS * 4;
 
 // Rows of a launch for K (padded) of kp: a multiple of TM.
 static int row_chunk(int M, size_t kp) {
@@ -790,15 +858,15 @@ static int row_chunk(int M, size_t kp) {
 size_t dgemm_tc_workspace(int M, int N, int K) {
   const size_t np = (size_t)ceil_div(N, TN) * TN;
   const size_t kp = (size_t)ceil_div(std::min(std::max(K, 1), KCHUNK), DKB) * DKB;
-  const size_t mp = row_chunk(M, kp);
-  return align256(mp * kp * DS * 2) + align256(np * kp * DS * 2) + align256(mp * 4) +
-         align256(np * 4) + align256(kSplitBytes);
+  const size_t mp = row_chunk(M, kp), passes = ceil_div(kp, KPASS);
+  return align256(mp * kp * DS * 2) + align256(np * kp * DS * 2) + align256(mp * 4 * passes) +
+         align256(np * 4 * passes) + align256(kSplitBytes);
 }
 
 size_t dgemm_tc_columns_bytes(int rows, int K) {
   const size_t np = (size_t)ceil_div(rows, TN) * TN;
   const size_t kp = (size_t)ceil_div(std::max(K, 1), DKB) * DKB;
-  return align256(np * kp * DS * 2) + align256(np * 4 * ceil_div(std::max(K, 1), KCHUNK));
+  return align256(np * kp * DS * 2) + align256(np * 4 * ceil_div(kp, KPASS));
 }
 
 int dgemm_tc_slice_columns(corr_context* c, const MatView& v, int rows, int K, void* ws,
@@ -809,7 +877,7 @@ int dgemm_tc_slice_columns(corr_context* c, const MatView& v, int rows, int K, v
   int* e = reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + align256(np * kp * DS * 2));
   for (int k0 = 0, p = 0; k0 < K; k0 += KCHUNK, ++p) {
     const int kn = std::min(KCHUNK, K - k0);
-    CORR_TRY(slice_operand<TN>(c, v, 0, rows, np, k0, kn, ceil_div(kn, DKB), e + (size_t)p * np,
+    CORR_TRY(slice_operand<TN>(c, v, 0, rows, np, k0, kn, ceil_div(kn, DKB), e + (size_t)p * PASSES * np,
                                planes + (size_t)p * KCHUNK * np * DS));
   }
   out->planes = planes;
@@ -827,15 +895,17 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
   uint16_t* Ad = reinterpret_cast<uint16_t*>(w);
   w += align256((size_t)mp * kp * DS * 2);
   int* ea = reinterpret_cast<int*>(w);
-  w += align256((size_t)mp * 4);
+  const size_t passes = ceil_div(kp, KPASS);
+  w += align256((size_t)mp * 4 * passes);
   uint16_t* Bw = reinterpret_cast<uint16_t*>(w);
   if (!g.pre) w += align256((size_t)np * kp * DS * 2);
   int* ebw = reinterpret_cast<int*>(w);
-  if (!g.pre) w += align256((size_t)np * 4);
+  if (!g.pre) w += align256((size_t)np * 4 * passes);
   static bool attr[64] = {};
   if (c->device < 0 || c->device >= 64 || !attr[c->device]) {
-    CORR_CUDA(cudaFuncSetAttribute(dgemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kDgSmem));
+    for (auto k : {dgemm_tc_kernel<false>, dgemm_tc_kernel<true>})
+      CORR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kDgSmem));
     if (c->device >= 0 && c->device < 64) attr[c->device] = true;
   }
   const int chunks = std::max(1, ceil_div(g.K, KCHUNK));
@@ -852,7 +922,7 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
       CORR_CUDA(cudaMemsetAsync(ebw, 0, (size_t)np * 4, c->stream));
     } else if (g.pre) {
       Bd = g.pre->planes + ((size_t)p * KCHUNK * g.pre->rows_pad + (size_t)g.col0 * nkb * DKB) * DS;
-      eb = g.pre->e + (size_t)p * g.pre->rows_pad + g.col0;
+      eb = g.pre->e + (size_t)p * PASSES * g.pre->rows_pad + g.col0;
     } else {
       CORR_TRY(slice_operand<TN>(c, g.B, 0, g.N, np, k0, kn, nkb, ebw, Bw));
     }
@@ -861,11 +931,11 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
       const long long tiles = (long long)mtn * ntn;
       const int parts = mp >= g.M && kn > 0 ? k_parts(tiles, nkb) : 1;
       unsigned long long* part_hi = reinterpret_cast<unsigned long long*>(w);
-      float* part_tail = reinterpret_cast<float*>(part_hi + kMaxSplitUnits * TM * TN);
-      unsigned* ticket = reinterpret_cast<unsigned*>(part_tail + kMaxSplitUnits * TM * TN);
+      float* part_tail = reinterpret_cast<float*>(part_hi + kMaxSplitSlots * TM * TN);
+      unsigned* ticket = reinterpret_cast<unsigned*>(part_tail + kMaxSplitSlots * TM * TN);
       if (kn > 0) {
         CORR_TRY(slice_operand<TM>(c, g.A, m0, rows, mtn * TM, k0, kn, nkb, ea, Ad, ticket,
-                                   parts > 1 ? (int)tiles * EWARPS : 0));
+                                   parts > 1 ? (int)tiles * (PASSES + 1) * EWARPS : 0));
       } else {
         CORR_CUDA(cudaMemsetAsync(Ad, 0, (size_t)mp * kp * DS * 2, c->stream));
         CORR_CUDA(cudaMemsetAsync(ea, 0, (size_t)mp * 4, c->stream));
@@ -875,6 +945,8 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
       a.Bd = Bd;
       a.ea = ea;
       a.eb = eb;
+      a.lea = mtn * TM;
+      a.leb = g.pre ? g.pre->rows_pad : np;
       a.C = g.C;
       a.alpha = g.alpha;
       a.scaled = pow2 ? 0 : 1;
@@ -893,12 +965,16 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
       a.accumulate = (g.accumulate || p > 0) ? 1 : 0;
       a.nsplit = parts;
       a.kper = ceil_div(nkb, parts);
+      a.nslot = parts + ceil_div(nkb, PASS_KB) - 1;
       a.part_hi = part_hi;
       a.part_tail = part_tail;
       a.ticket = ticket;
+      a.tiles = (int)tiles;
       a.total = tiles * a.nsplit;
       const int grid = (int)std::min<long long>(a.total, c->sms - c->spare_sms);
-      dgemm_tc_kernel<<<grid, NTHREADS, kDgSmem, c->stream>>>(a, &c->dres->status);
+      (parts > 1 ? dgemm_tc_kernel<true> : dgemm_tc_kernel<false>)<<<grid, NTHREADS, kDgSmem,
+                                                                  c->stream>>>(
+          a, &c->dres->status);
       CORR_CUDA(cudaGetLastError());
       c->launches += 1;
     }

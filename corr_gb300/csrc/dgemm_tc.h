@@ -42,7 +42,7 @@ struct DgColumns {
 // n < N, k < K.  a_lower: A(m, k) == 0 for k > m (skipped).  Inputs finite;
 // in a plain-form call (corr_context::digit_guard) an operand with a value
 // outside the splitting's range (not finite, or a row whose largest magnitude
-// is below 2^-958) raises kStatusNeedFp64 in the context's status word.
+// in 512 of K is below 2^-958) raises kStatusNeedFp64 in the context's status word.
 struct DgemmTc {
   MatView A, B;
   OutView C;
