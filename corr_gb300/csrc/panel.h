@@ -26,7 +26,7 @@ struct PanelPlan {
 constexpr size_t kPanelBudget = (size_t)512 << 20;
 PanelPlan panel_plan(int o, int v, int X, size_t budget);
 
-// panel = B_block^T B over Q; cols: the sliced columns of B.  dws:
+// panel = B_block^T B over Q, its diagonal (ia|ia) in FP64; cols: the sliced columns of B.  dws:
 // dgemm_tc_workspace(ni v, kDgColTile, X) bytes.
 int panel_product(corr_context* c, int o, int v, int X, const double* bia, const DgColumns& cols,
                   int i0, int ni, double* panel, void* dws, PanelView* pv);
