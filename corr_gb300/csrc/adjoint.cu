@@ -254,7 +254,8 @@ size_t rimp2_gradient_tc_workspace(int o, int v, int X, size_t panel_budget) {
 
 int rimp2_gradient_tc(corr_context* c, Carver& w, int o, int v, int X, const double* bia,
                       const double* eps, double* dbia, double* deps, size_t panel_budget) {
-  CORR_CHECK_ARG(v <= 6144, "corr_rimp2_gradient_tc: nvir %d above 6144", v);
+  CORR_CHECK_ARG(v <= kPanelMaxNvir, "corr_rimp2_gradient_tc: nvir %d above %d", v,
+                 kPanelMaxNvir);
   const PanelPlan p = panel_plan(o, v, X, panel_budget);
   const int R = o * v;
   double* panel = static_cast<double*>(w.take(p.panel_bytes));
@@ -364,7 +365,7 @@ extern "C" int corr_rimp2_gradient(corr_context* c, int nocc, int nvir, int naux
   // overlaps an input, or nvir is beyond that form's limit)
   const size_t nb = (size_t)std::max(nocc, 0) * std::max(nvir, 0) * std::max(naux, 0) * 8;
   const size_t ne = ((size_t)std::max(nocc, 0) + std::max(nvir, 0)) * 8;
-  const bool fp64_only = nvir > 6144 || nocc > 16384 || overlaps(dbia, nb, bia, nb) ||
+  const bool fp64_only = nvir > kPanelMaxNvir || nocc > 16384 || overlaps(dbia, nb, bia, nb) ||
                          overlaps(deps, ne, eps, ne) || overlaps(dbia, nb, eps, ne) ||
                          overlaps(deps, ne, bia, nb);
   return with_fp64_retry(c, fp64_only, [&]() -> int {

@@ -269,10 +269,15 @@ int panel_product(corr_context* c, int o, int v, int X, const double* bia, const
 int launch_panel(corr_context* c, const PanelView& pv, const double* eps, double* deps,
                  double* part, int split, bool grad) {
   const dim3 grid((unsigned)(pv.ni * (pv.o - pv.i0)), (unsigned)split);
-  // the W sums of a long virtual range go beyond the 48 KB that need no opt-in
-  if (grad && pv.v > 4096)
+  // The W sums of a long virtual range go beyond the 48 KB that need no opt-in.  The
+  // limit belongs to the kernel, not to a context: it is set to the largest nvir's,
+  // the same for every caller.
+  static bool attr[64] = {};
+  if (grad && (c->device < 0 || c->device >= 64 || !attr[c->device])) {
     CORR_CUDA(cudaFuncSetAttribute(panel_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   pv.v * 8));
+                                   kPanelMaxNvir * 8));
+    if (c->device >= 0 && c->device < 64) attr[c->device] = true;
+  }
   if (grad)
     panel_kernel<true><<<grid, 256, (size_t)pv.v * 8, c->stream>>>(pv, eps, deps, part);
   else

@@ -24,6 +24,7 @@ struct PanelPlan {
   long long partials;
 };
 constexpr size_t kPanelBudget = (size_t)512 << 20;
+constexpr int kPanelMaxNvir = 6144;  // of the gradient's panels (sums of W in shared memory)
 PanelPlan panel_plan(int o, int v, int X, size_t budget);
 
 // panel = B_block^T B over Q, its diagonal (ia|ia) in FP64; cols: the sliced columns of B.  dws:
