@@ -239,16 +239,15 @@ size_t rimp2_gradient_workspace(int o, int v, int sms, size_t panel_budget) {
 //   dB[Q][(i, a)] += 2 sum_(j,b) G[(i, a)][(j, b)] B[Q][(j, b)]   (j >= i0),
 //   dB[Q][(j, b)] += 2 sum_(i,a) G[(i, a)][(j, b)] B[Q][(i, a)]   (j beyond I),
 // the second by G^{ji}_ba = G^{ij}_ab: (ia|jb) is formed for half of the pairs.
-static size_t gradient_product_workspace(int o, int v, int X, int ni) {
+static size_t gradient_product_workspace(int o, int v, int X, const PanelPlan& p) {
   const int R = o * v;
-  return std::max(std::max(dgemm_tc_workspace(ni * v, kDgColTile, X),
-                           dgemm_tc_workspace(X, ni * v, R)),
-                  dgemm_tc_workspace(X, R, ni * v));
+  return std::max(std::max(p.product_bytes, dgemm_tc_workspace(X, p.ni * v, R)),
+                  dgemm_tc_workspace(X, R, p.ni * v));
 }
 
 size_t rimp2_gradient_tc_workspace(int o, int v, int X, size_t panel_budget) {
   const PanelPlan p = panel_plan(o, v, X, panel_budget);
-  return p.panel_bytes + p.col_bytes + gradient_product_workspace(o, v, X, p.ni) +
+  return p.panel_bytes + p.col_bytes + gradient_product_workspace(o, v, X, p) +
          (size_t)p.partials * 16 + (size_t)kReduceBlocks * 16 + 8 * 256;
 }
 
@@ -260,19 +259,20 @@ int rimp2_gradient_tc(corr_context* c, Carver& w, int o, int v, int X, const dou
   const int R = o * v;
   double* panel = static_cast<double*>(w.take(p.panel_bytes));
   void* cws = w.take(p.col_bytes);
-  void* dws = w.take(gradient_product_workspace(o, v, X, p.ni));
+  void* dws = w.take(gradient_product_workspace(o, v, X, p));
   double* part = static_cast<double*>(w.take((size_t)p.partials * 16));
   unsigned* ticket = static_cast<unsigned*>(w.take(16));
   double* scratch = static_cast<double*>(w.take((size_t)kReduceBlocks * 16));
   CORR_CUDA(cudaMemsetAsync(deps, 0, (size_t)(o + v) * 8, c->stream));
   DgColumns cols;
-  CORR_TRY(dgemm_tc_slice_columns(c, mat_view(bia, 1, R), R, X, cws, &cols));
+  if (p.col_bytes) CORR_TRY(dgemm_tc_slice_columns(c, mat_view(bia, 1, R), R, X, cws, &cols));
   long long np = 0;
   for (int i0 = 0; i0 < o; i0 += p.ni) {
     const int ni = std::min(p.ni, o - i0);
     const long long r0 = (long long)i0 * v, r1 = (long long)(i0 + ni) * v;
     PanelView pv;
-    CORR_TRY(panel_product(c, o, v, X, bia, cols, i0, ni, panel, dws, &pv));
+    CORR_TRY(panel_product(c, o, v, X, bia, p.col_bytes ? &cols : nullptr, i0, ni, panel, dws,
+                           &pv));
     CORR_TRY(launch_panel(c, pv, eps, deps, part + 2 * np, p.split, true));
     np += (long long)ni * (o - i0) * p.split;
     DgemmTc d;

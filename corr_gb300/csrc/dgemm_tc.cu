@@ -71,9 +71,6 @@ constexpr int KPASS = 512;                // K per pass (exact levels 0..5)
 constexpr int KCHUNK = 2048;              // K per launch (digit planes in the workspace)
 constexpr int PASS_KB = KPASS / DKB;
 constexpr int PASSES = KCHUNK / KPASS;    // scales per row and launch
-// Rows per launch: the row operand's digit planes stay below about 1 GiB (at
-// least 256 row tiles, so that a narrow product still fills the SMs).
-constexpr size_t kRowPlaneBytes = (size_t)1 << 30;
 constexpr int A_PLANE = TM * DKB * 2;     // 8 KB
 constexpr int B_PLANE = TN * DKB * 2;     // 4 KB
 constexpr int A_BYTES = DS * A_PLANE;     // 64 KB
@@ -849,18 +846,29 @@ static int k_parts(long long tiles, int nkb) {
 constexpr size_t kSplitBytes = (size_t)kMaxSplitSlots * TM * TN * 12 +
                                kMaxSplitSlots * (PASSES + 1) * EWARPS * 4;
 
-// Rows of a launch for K (padded) of kp: a multiple of TM.
-static int row_chunk(int M, size_t kp) {
-  const size_t fit = kRowPlaneBytes / (kp * DS * 2) / TM * TM;
-  return (int)std::min<size_t>((size_t)ceil_div(M, TM) * TM, std::max<size_t>(fit, 256 * TM));
+// Rows (columns) of a launch for K (padded) of kp, a multiple of the tile: an
+// operand's digit planes stay within kDgPlaneBytes (at least 256 tiles, so that a
+// narrow product still fills the SMs).
+static int plane_chunk(int rows, size_t kp, int tile) {
+  const size_t fit = kDgPlaneBytes / (kp * DS * 2) / tile * tile;
+  return (int)std::min<size_t>((size_t)ceil_div(rows, tile) * tile,
+                               std::max<size_t>(fit, 256 * tile));
+}
+
+// Bytes of an operand's planes and exponents in any launch of plane_chunk(rows, kp,
+// tile) rows; no less for a larger kp, so that a workspace also holds the products
+// with a smaller K.
+static size_t operand_bytes(int rows, size_t kp, int tile) {
+  const size_t rp = (size_t)ceil_div(rows, tile) * tile, row = kp * DS * 2;
+  const size_t planes = std::min(rp * row, std::max(kDgPlaneBytes, 256 * tile * row));
+  // kp >= 32: an exponent per 512 of k is at most 1/64 of the planes
+  const size_t exps = std::min(rp * 4 * ceil_div(kp, KPASS), planes / 64 + 4096);
+  return align256(planes) + align256(exps);
 }
 
 size_t dgemm_tc_workspace(int M, int N, int K) {
-  const size_t np = (size_t)ceil_div(N, TN) * TN;
   const size_t kp = (size_t)ceil_div(std::min(std::max(K, 1), KCHUNK), DKB) * DKB;
-  const size_t mp = row_chunk(M, kp), passes = ceil_div(kp, KPASS);
-  return align256(mp * kp * DS * 2) + align256(np * kp * DS * 2) + align256(mp * 4 * passes) +
-         align256(np * 4 * passes) + align256(kSplitBytes);
+  return operand_bytes(M, kp, TM) + operand_bytes(N, kp, TN) + align256(kSplitBytes);
 }
 
 size_t dgemm_tc_columns_bytes(int rows, int K) {
@@ -888,9 +896,9 @@ int dgemm_tc_slice_columns(corr_context* c, const MatView& v, int rows, int K, v
 
 int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
   if (g.M <= 0 || g.N <= 0) return CORR_OK;
-  const int ntn = ceil_div(g.N, TN), np = ntn * TN;
   const size_t kp = (size_t)ceil_div(std::min(std::max(g.K, 1), KCHUNK), DKB) * DKB;
-  const int mp = row_chunk(g.M, kp);
+  const int mp = plane_chunk(g.M, kp, TM);
+  const int np = g.pre ? ceil_div(g.N, TN) * TN : plane_chunk(g.N, kp, TN);
   uint8_t* w = static_cast<uint8_t*>(ws);
   uint16_t* Ad = reinterpret_cast<uint16_t*>(w);
   w += align256((size_t)mp * kp * DS * 2);
@@ -915,68 +923,73 @@ int dgemm_tc(corr_context* c, const DgemmTc& g, void* ws) {
   for (int p = 0; p < chunks; ++p) {
     const int k0 = p * KCHUNK, kn = std::min(KCHUNK, g.K - k0);
     const int nkb = ceil_div(std::max(kn, 1), DKB);
-    const uint16_t* Bd = Bw;
-    const int* eb = ebw;
-    if (kn <= 0) {  // K == 0: zero digits give C = 0 (or C unchanged when accumulating)
-      CORR_CUDA(cudaMemsetAsync(Bw, 0, (size_t)np * kp * DS * 2, c->stream));
-      CORR_CUDA(cudaMemsetAsync(ebw, 0, (size_t)np * 4, c->stream));
-    } else if (g.pre) {
-      Bd = g.pre->planes + ((size_t)p * KCHUNK * g.pre->rows_pad + (size_t)g.col0 * nkb * DKB) * DS;
-      eb = g.pre->e + (size_t)p * PASSES * g.pre->rows_pad + g.col0;
-    } else {
-      CORR_TRY(slice_operand<TN>(c, g.B, 0, g.N, np, k0, kn, nkb, ebw, Bw));
-    }
-    for (int m0 = 0; m0 < g.M; m0 += mp) {
-      const int rows = std::min(mp, g.M - m0), mtn = ceil_div(rows, TM);
-      const long long tiles = (long long)mtn * ntn;
-      const int parts = mp >= g.M && kn > 0 ? k_parts(tiles, nkb) : 1;
-      unsigned long long* part_hi = reinterpret_cast<unsigned long long*>(w);
-      float* part_tail = reinterpret_cast<float*>(part_hi + kMaxSplitSlots * TM * TN);
-      unsigned* ticket = reinterpret_cast<unsigned*>(part_tail + kMaxSplitSlots * TM * TN);
-      if (kn > 0) {
-        CORR_TRY(slice_operand<TM>(c, g.A, m0, rows, mtn * TM, k0, kn, nkb, ea, Ad, ticket,
-                                   parts > 1 ? (int)tiles * (PASSES + 1) * EWARPS : 0));
+    for (int n0 = 0; n0 < g.N; n0 += np) {
+      const int cols = std::min(np, g.N - n0), ntn = ceil_div(cols, TN);
+      const uint16_t* Bd = Bw;
+      const int* eb = ebw;
+      if (kn <= 0) {  // K == 0: zero digits give C = 0 (or C unchanged when accumulating)
+        CORR_CUDA(cudaMemsetAsync(Bw, 0, (size_t)np * kp * DS * 2, c->stream));
+        CORR_CUDA(cudaMemsetAsync(ebw, 0, (size_t)np * 4, c->stream));
+      } else if (g.pre) {
+        Bd = g.pre->planes +
+             ((size_t)p * KCHUNK * g.pre->rows_pad + (size_t)g.col0 * nkb * DKB) * DS;
+        eb = g.pre->e + (size_t)p * PASSES * g.pre->rows_pad + g.col0;
       } else {
-        CORR_CUDA(cudaMemsetAsync(Ad, 0, (size_t)mp * kp * DS * 2, c->stream));
-        CORR_CUDA(cudaMemsetAsync(ea, 0, (size_t)mp * 4, c->stream));
+        CORR_TRY(slice_operand<TN>(c, g.B, n0, cols, ntn * TN, k0, kn, nkb, ebw, Bw));
       }
-      DgArgs a;
-      a.Ad = Ad;
-      a.Bd = Bd;
-      a.ea = ea;
-      a.eb = eb;
-      a.lea = mtn * TM;
-      a.leb = g.pre ? g.pre->rows_pad : np;
-      a.C = g.C;
-      a.alpha = g.alpha;
-      a.scaled = pow2 ? 0 : 1;
-      a.alpha_exp = pow2 ? ax - 1 : 0;
-      a.sign = pow2 && g.alpha < 0.0 ? 0x80000000u : 0u;
-      a.M = m0 + rows;
-      a.N = g.N;
-      a.m0 = m0;
-      a.nkb = nkb;
-      a.mtn = mtn;
-      a.ntn = ntn;
-      // keep the larger operand's tile shared by adjacent units (L2 reuse)
-      a.col_major_order = ntn * TN > mtn * TM ? 1 : 0;
-      a.a_lower = g.a_lower ? 1 : 0;
-      a.k0 = k0;
-      a.accumulate = (g.accumulate || p > 0) ? 1 : 0;
-      a.nsplit = parts;
-      a.kper = ceil_div(nkb, parts);
-      a.nslot = parts + ceil_div(nkb, PASS_KB) - 1;
-      a.part_hi = part_hi;
-      a.part_tail = part_tail;
-      a.ticket = ticket;
-      a.tiles = (int)tiles;
-      a.total = tiles * a.nsplit;
-      const int grid = (int)std::min<long long>(a.total, c->sms - c->spare_sms);
-      (parts > 1 ? dgemm_tc_kernel<true> : dgemm_tc_kernel<false>)<<<grid, NTHREADS, kDgSmem,
-                                                                  c->stream>>>(
-          a, &c->dres->status);
-      CORR_CUDA(cudaGetLastError());
-      c->launches += 1;
+      for (int m0 = 0; m0 < g.M; m0 += mp) {
+        const int rows = std::min(mp, g.M - m0), mtn = ceil_div(rows, TM);
+        const long long tiles = (long long)mtn * ntn;
+        const int parts = mp >= g.M && np >= g.N && kn > 0 ? k_parts(tiles, nkb) : 1;
+        unsigned long long* part_hi = reinterpret_cast<unsigned long long*>(w);
+        float* part_tail = reinterpret_cast<float*>(part_hi + kMaxSplitSlots * TM * TN);
+        unsigned* ticket = reinterpret_cast<unsigned*>(part_tail + kMaxSplitSlots * TM * TN);
+        if (kn <= 0) {
+          CORR_CUDA(cudaMemsetAsync(Ad, 0, (size_t)mp * kp * DS * 2, c->stream));
+          CORR_CUDA(cudaMemsetAsync(ea, 0, (size_t)mp * 4, c->stream));
+        } else if (n0 == 0 || mp < g.M) {  // else the planes of all rows are there
+          CORR_TRY(slice_operand<TM>(c, g.A, m0, rows, mtn * TM, k0, kn, nkb, ea, Ad, ticket,
+                                     parts > 1 ? (int)tiles * (PASSES + 1) * EWARPS : 0));
+        }
+        DgArgs a;
+        a.Ad = Ad;
+        a.Bd = Bd;
+        a.ea = ea;
+        a.eb = eb;
+        a.lea = mtn * TM;
+        a.leb = g.pre ? g.pre->rows_pad : ntn * TN;
+        a.C = g.C;
+        a.C.p += (long long)n0 * g.C.cs;
+        a.alpha = g.alpha;
+        a.scaled = pow2 ? 0 : 1;
+        a.alpha_exp = pow2 ? ax - 1 : 0;
+        a.sign = pow2 && g.alpha < 0.0 ? 0x80000000u : 0u;
+        a.M = m0 + rows;
+        a.N = cols;
+        a.m0 = m0;
+        a.nkb = nkb;
+        a.mtn = mtn;
+        a.ntn = ntn;
+        // keep the larger operand's tile shared by adjacent units (L2 reuse)
+        a.col_major_order = ntn * TN > mtn * TM ? 1 : 0;
+        a.a_lower = g.a_lower ? 1 : 0;
+        a.k0 = k0;
+        a.accumulate = (g.accumulate || p > 0) ? 1 : 0;
+        a.nsplit = parts;
+        a.kper = ceil_div(nkb, parts);
+        a.nslot = parts + ceil_div(nkb, PASS_KB) - 1;
+        a.part_hi = part_hi;
+        a.part_tail = part_tail;
+        a.ticket = ticket;
+        a.tiles = (int)tiles;
+        a.total = tiles * a.nsplit;
+        const int grid = (int)std::min<long long>(a.total, c->sms - c->spare_sms);
+        (parts > 1 ? dgemm_tc_kernel<true> : dgemm_tc_kernel<false>)<<<grid, NTHREADS, kDgSmem,
+                                                                    c->stream>>>(
+            a, &c->dres->status);
+        CORR_CUDA(cudaGetLastError());
+        c->launches += 1;
+      }
     }
   }
   return CORR_OK;

@@ -56,6 +56,9 @@ struct DgemmTc {
   int col0 = 0;
 };
 constexpr int kDgColTile = 64;
+// Digit planes of an operand at a time (16 bytes per element); a product whose
+// operand takes more runs in blocks of its rows or columns.
+constexpr size_t kDgPlaneBytes = (size_t)1 << 30;
 
 // Device workspace of one dgemm_tc call (bytes).
 size_t dgemm_tc_workspace(int M, int N, int K);

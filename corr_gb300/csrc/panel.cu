@@ -228,6 +228,8 @@ PanelPlan panel_plan(int o, int v, int X, size_t budget) {
   p.ni = (int)std::max<size_t>(1, std::min<size_t>(o, budget / per_i));
   p.panel_bytes = per_i * p.ni;
   p.col_bytes = dgemm_tc_columns_bytes(o * v, X);
+  if (p.col_bytes > kDgPlaneBytes + kDgPlaneBytes / 64) p.col_bytes = 0;  // (with the exponents)
+  p.product_bytes = dgemm_tc_workspace(p.ni * v, p.col_bytes ? kDgColTile : o * v, X);
   long long n = 0;
   for (int i0 = 0; i0 < o; i0 += p.ni) n += (long long)std::min(p.ni, o - i0) * (o - i0);
   // CTAs per (i, j) block: one per column of tiles while that is a few million
@@ -237,7 +239,7 @@ PanelPlan panel_plan(int o, int v, int X, size_t budget) {
   return p;
 }
 
-int panel_product(corr_context* c, int o, int v, int X, const double* bia, const DgColumns& cols,
+int panel_product(corr_context* c, int o, int v, int X, const double* bia, const DgColumns* cols,
                   int i0, int ni, double* panel, void* dws, PanelView* pv) {
   const int R = o * v;
   pv->p = panel;
@@ -249,7 +251,7 @@ int panel_product(corr_context* c, int o, int v, int X, const double* bia, const
   pv->ni = ni;
   DgemmTc m;
   m.A = mat_view(bia + (size_t)i0 * v, 1, R);  // rows (i, a) of the block, over Q
-  m.B = mat_view(bia, 1, R);
+  m.B = mat_view(bia + pv->col0, 1, R);
   m.C = out_view(panel, pv->ld, 1);
   m.M = ni * v;
   m.N = (int)pv->ld;
@@ -257,7 +259,7 @@ int panel_product(corr_context* c, int o, int v, int X, const double* bia, const
   m.alpha = 1.0;
   m.accumulate = false;
   m.a_lower = false;
-  m.pre = &cols;
+  m.pre = cols;
   m.col0 = (int)pv->col0;
   CORR_TRY(dgemm_tc(c, m, dws));
   panel_diag_kernel<<<(unsigned)(((long long)ni * v + 31) / 32), 1024, 0, c->stream>>>(*pv, bia, X);
@@ -292,7 +294,7 @@ size_t energy_panel_bytes(int o, int v, int X) {
   Carver w{nullptr, 0};
   w.take(p.panel_bytes);
   w.take(p.col_bytes);
-  w.take(dgemm_tc_workspace(p.ni * v, kDgColTile, X));
+  w.take(p.product_bytes);
   w.take((size_t)p.partials * 16);
   w.take(16);
   w.take((size_t)kReduceBlocks * 16);
@@ -304,17 +306,19 @@ int energy_from_panels(corr_context* c, Carver& w, int o, int v, int X, const do
   const PanelPlan p = panel_plan(o, v, X, kPanelBudget);
   double* panel = static_cast<double*>(w.take(p.panel_bytes));
   void* cws = w.take(p.col_bytes);
-  void* dws = w.take(dgemm_tc_workspace(p.ni * v, kDgColTile, X));
+  void* dws = w.take(p.product_bytes);
   double* part = static_cast<double*>(w.take((size_t)p.partials * 16));
   unsigned* ticket = static_cast<unsigned*>(w.take(16));
   double* scratch = static_cast<double*>(w.take((size_t)kReduceBlocks * 16));
   DgColumns cols;
-  CORR_TRY(dgemm_tc_slice_columns(c, mat_view(bia, 1, (long long)o * v), o * v, X, cws, &cols));
+  if (p.col_bytes)
+    CORR_TRY(dgemm_tc_slice_columns(c, mat_view(bia, 1, (long long)o * v), o * v, X, cws, &cols));
   long long np = 0;
   for (int i0 = 0; i0 < o; i0 += p.ni) {
     const int ni = std::min(p.ni, o - i0);
     PanelView pv;
-    CORR_TRY(panel_product(c, o, v, X, bia, cols, i0, ni, panel, dws, &pv));
+    CORR_TRY(panel_product(c, o, v, X, bia, p.col_bytes ? &cols : nullptr, i0, ni, panel, dws,
+                           &pv));
     CORR_TRY(launch_panel(c, pv, eps, nullptr, part + 2 * np, p.split, false));
     np += (long long)ni * (o - i0) * p.split;
   }

@@ -16,20 +16,22 @@ struct PanelView {
 };
 
 // Blocks of ni occupied orbitals whose panels stay within `budget` (at least
-// one orbital), the column operand's digit planes, and the partials of all
-// launch_panel calls.
+// one orbital), the column operand's digit planes (col_bytes; 0 where they would
+// exceed kDgPlaneBytes: every block's product slices its columns again, 24 bytes
+// of traffic per element against 2 ni nvir operations at the digit GEMM's rate),
+// the workspace of a block's product, and the partials of all launch_panel calls.
 struct PanelPlan {
   int ni, split;
-  size_t panel_bytes, col_bytes;
+  size_t panel_bytes, col_bytes, product_bytes;
   long long partials;
 };
 constexpr size_t kPanelBudget = (size_t)512 << 20;
 constexpr int kPanelMaxNvir = 6144;  // of the gradient's panels (sums of W in shared memory)
 PanelPlan panel_plan(int o, int v, int X, size_t budget);
 
-// panel = B_block^T B over Q, its diagonal (ia|ia) in FP64; cols: the sliced columns of B.  dws:
-// dgemm_tc_workspace(ni v, kDgColTile, X) bytes.
-int panel_product(corr_context* c, int o, int v, int X, const double* bia, const DgColumns& cols,
+// panel = B_block^T B over Q, its diagonal (ia|ia) in FP64; cols: the sliced columns of B, or null.
+// dws: product_bytes of the plan.
+int panel_product(corr_context* c, int o, int v, int X, const double* bia, const DgColumns* cols,
                   int i0, int ni, double* panel, void* dws, PanelView* pv);
 // Energy partials ({E_OS, E_SS} per CTA), or with grad the elements replaced by
 // the adjoint G, W added to deps and {E, 0} partials.  split (of the plan): CTAs
