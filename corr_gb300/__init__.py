@@ -182,6 +182,14 @@ class Context:
         status CORR_ERR_DEVICE_TIMEOUT; the context stays usable)."""
         check(self._L.corr_selftest_wait_timeout(self._h, int(limit_ms)))
 
+    def selftest_fp64(self, function, x):
+        """1 / x ("recip") or x^-1/2 ("rsqrt") of a float64 array, by the FP64
+        functions of the kernels."""
+        out = self._out(x, tuple(x.shape), None)
+        check(self._L.corr_selftest_fp64(self._h, {"recip": 0, "rsqrt": 1}[function], x.size,
+                                         _ptr(x), _ptr(out)))
+        return out
+
     def set_fp64_strict(self, strict=True):
         """Plain-form calls on the FP64 pipe only (True), or with the panels of
         large "fp64" energies, the gradient and the metric on the FP64-accurate

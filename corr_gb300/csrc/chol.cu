@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "dgemm_tc.h"
+#include "fp64_approx.cuh"
 #include "gemm_fp64.h"
 #include "kernels.h"
 
@@ -48,15 +49,6 @@ __global__ void chol_init(const double* __restrict__ J, int m, double shift,
     A[e] = J[e] - (x == y ? shift : 0.0);
     Lm[e] = 0.0;
   }
-}
-
-// 1 / d for a positive normal pivot: the hardware's 20-bit estimate and one
-// cubic Newton step (three dependent FP64 instructions on the critical path).
-__device__ __forceinline__ double recip_pivot(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
 }
 
 // One CTA: factor the nb x nb diagonal block at (k, k) of A (lower triangle
@@ -103,7 +95,7 @@ __global__ void __launch_bounds__(256) chol_diag(const double* __restrict__ A, i
       pd = 1.0;
       bad = 1;
     }
-    pr = ex < 0x7FD ? recip_pivot(pd) : 1.0 / pd;
+    pr = recip64(pd);
   };
   __syncthreads();
   if (warp == 0) pivot(m0[0], 0);

@@ -35,6 +35,7 @@
 
 #include "abi_internal.h"
 #include "common.cuh"
+#include "fp64_approx.cuh"
 
 namespace corr {
 
@@ -88,9 +89,10 @@ __host__ __device__ constexpr int tuv_index(int t, int u, int v) {
 // 1/16, |dT| <= 1/32, truncation below 2^-55 relative) and downward
 // recursion F_n = (2T F_{n+1} + e^-T) / (2n + 1), with e^-T from the grid
 // point's and an 8-term exponential series of the offset (below 2^-55); above,
-// the asymptotic F_0 = sqrt(pi/T) / 2 (erf(sqrt T) = 1 to 1e-18) and upward
-// recursion without the e^-T term (below 4e-18 relative).  The tables hold the
-// Taylor coefficients F_{n+k} / k!, one FMA per term.
+// the asymptotic F_0 = sqrt(pi/T) / 2 and upward recursion without the e^-T term:
+// what they leave out, e^-T / (2T) (1 + (2n+1) / (2T) + ...), is below 7e-20 (at
+// T = 40, 4e-19 of F_0 and 7e-11 of F_7, which is 9e-10 there).  The tables hold
+// the Taylor coefficients F_{n+k} / k!, one FMA per term.
 constexpr int kBoysOrders = 16;                // tabulated n = 0..15
 constexpr int kBoysTerms = 8;
 constexpr int kBoysMax = kBoysOrders - kBoysTerms;  // highest NMAX
@@ -326,17 +328,6 @@ __global__ void __launch_bounds__(128) e_table_kernel(Basis3 g) {
         }
     }
   }
-}
-
-// d^-1/2: the hardware's 20-bit estimate and one cubic step of Newton's method,
-// r <- r + r e (1/2 + 3/8 e) with e = 1 - d r^2, five FP64 instructions.
-__device__ __forceinline__ double rsqrt64(double d) {
-  const int ex = (__double2hiint(d) >> 20) & 0x7FF;
-  if (ex < 2 || ex > 2044) return rsqrt(d);
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d * r, r, 1.0);
-  return fma(r * e, fma(0.375, e, 0.5), r);
 }
 
 // gamma p / (gamma + p), and 2 pi^(5/2) / (p gamma sqrt(p + gamma)) times the

@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "dgemm_tc.h"
+#include "fp64_approx.cuh"
 #include "kernels.h"
 #include "panel.h"
 
@@ -21,19 +22,6 @@ namespace corr {
 namespace {
 
 constexpr int PT = 32;  // tile edge
-
-// 1 / d: the hardware's 20-bit estimate and one cubic step of Newton's method,
-// r <- r + r (e + e^2) with e = 1 - d r, three FP64 instructions for the
-// division's eight or more (the FP64 pipe bounds this kernel).  Zero,
-// subnormal, infinite and NaN arguments take the division.
-__device__ __forceinline__ double recip64(double d) {
-  const int ex = (__double2hiint(d) >> 20) & 0x7FF;
-  if (ex < 2 || ex > 2044) return 1.0 / d;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
 
 // CTAs of an (i, j) block of the panel (blockIdx.x) share its columns of 32 x 32
 // tile pairs (A <= B, column B to blockIdx.y): with one CTA per block the 276

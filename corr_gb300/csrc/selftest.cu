@@ -1,13 +1,19 @@
-// Diagnostic: the bounded-wait path of the kernels, exercised on purpose.
+// Diagnostics.
 //
+// corr_selftest_wait_timeout: the bounded-wait path of the kernels, exercised on
+// purpose.
 // Every mbarrier wait of the tcgen05 kernels gives up after a time limit,
 // raises CORR_ERR_DEVICE_TIMEOUT in the call's status word and lets the CTA
 // wind down, so a lost arrival never hangs the GPU.  This entry point runs
 // that path: one CTA waits, with the same primitive, on an mbarrier phase that
 // nothing completes, for a caller-chosen limit.  No fault, trap or unbounded
 // loop is involved; the context stays usable afterwards.
+//
+// corr_selftest_fp64: the FP64 functions of fp64_approx.cuh, one argument per
+// thread.
 #include "abi_internal.h"
 #include "common.cuh"
+#include "fp64_approx.cuh"
 
 namespace corr {
 namespace {
@@ -22,6 +28,13 @@ __global__ void wait_selftest_kernel(unsigned long long limit_ns, int* status) {
   }
   __syncthreads();
   if (threadIdx.x == 0) mbar_wait_for(&bar, 0, &abort_flag, status, limit_ns);
+}
+
+__global__ void fp64_selftest_kernel(int which, long long n, const double* __restrict__ x,
+                                     double* __restrict__ out) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x)
+    out[k] = which ? rsqrt64(x[k]) : recip64(x[k]);
 }
 
 }  // namespace
@@ -41,6 +54,24 @@ int corr_selftest_wait_timeout(corr_context* c, int limit_ms) {
                                                 &c->dres->status);
   CORR_CUDA(cudaGetLastError());
   c->launches += 1;
+  return finish_results(c, 0);
+}
+
+int corr_selftest_fp64(corr_context* c, int which, long long n, const double* x, double* out) {
+  CORR_CHECK_ARG(c && x && out, "corr_selftest_fp64: null argument");
+  CORR_CHECK_ARG(n >= 1 && (which == 0 || which == 1), "corr_selftest_fp64: bad n or function");
+  CORR_CUDA(cudaSetDevice(c->device));
+  CORR_TRY(c->ws.reserve((size_t)n * 16 + 512));
+  Carver w{c->ws.ptr, 0};
+  void* slot = w.take((size_t)n * 8);
+  double* d_out = static_cast<double*>(w.take((size_t)n * 8));
+  CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
+  const double* d_x = static_cast<const double*>(stage_in(c, x, (size_t)n * 8, slot));
+  CORR_CHECK_ARG(d_x, "host-to-device copy failed");
+  fp64_selftest_kernel<<<c->sms * 4, 256, 0, c->stream>>>(which, n, d_x, d_out);
+  CORR_CUDA(cudaGetLastError());
+  c->launches += 1;
+  CORR_TRY(stage_out(c, out, d_out, (size_t)n * 8));
   return finish_results(c, 0);
 }
 

@@ -179,6 +179,10 @@ int corr_rimp2_energy_batched_async(corr_context* ctx, int n, const corr_rimp2_i
  * the context remains usable. */
 int corr_selftest_wait_timeout(corr_context* ctx, int limit_ms);
 
+/* Diagnostic: out[k] = 1 / x[k] (which = 0) or x[k]^-1/2 (which = 1), k < n, by
+ * the FP64 functions that the kernels use in place of the library's. */
+int corr_selftest_fp64(corr_context* ctx, int which, long long n, const double* x, double* out);
+
 /* Tile shape of the tcgen05 energy kernel (no counterpart in the reference).
  * Accepts 0 or 1 and has no effect: every tile runs 128 wide, the padded
  * columns of the last virtual tile being zeros.  (A narrower last tile needs
