@@ -190,6 +190,13 @@ class Context:
                                          _ptr(x), _ptr(out)))
         return out
 
+    def selftest_factor(self, J):
+        """(L, L^-1) of J = L L^T as the 3-index pipeline's precision forms
+        compute them."""
+        L, X = (self._out(J, tuple(J.shape), None) for _ in range(2))
+        check(self._L.corr_selftest_factor(self._h, J.shape[0], _ptr(J), _ptr(L), _ptr(X)))
+        return L, X
+
     def set_fp64_strict(self, strict=True):
         """Plain-form calls on the FP64 pipe only (True), or with the panels of
         large "fp64" energies, the gradient and the metric on the FP64-accurate

@@ -96,6 +96,7 @@ SIGNATURES = {
     "corr_set_fp64_strict": [_vp, _i],
     "corr_selftest_wait_timeout": [_vp, _i],
     "corr_selftest_fp64": [_vp, _i, _ll, _vp, _vp],
+    "corr_selftest_factor": [_vp, _i, _vp, _vp, _vp],
     "corr_rimp2_batch_autotune": [_vp, _i, ctypes.POINTER(RIMP2Instance), _i, ctypes.POINTER(_i),
                                   ctypes.POINTER(_i), ctypes.POINTER(_i),
                                   ctypes.POINTER(ctypes.c_float)],

@@ -11,11 +11,19 @@
 //
 // corr_selftest_fp64: the FP64 functions of fp64_approx.cuh, one argument per
 // thread.
+//
+// corr_selftest_factor: the Cholesky factor with its inverse (chol.cu) as the
+// precision forms of the 3-index pipeline take it, which otherwise shows only in
+// energies that their own digits limit to 1e-8.
 #include "abi_internal.h"
 #include "common.cuh"
+#include "dgemm_tc.h"
 #include "fp64_approx.cuh"
 
 namespace corr {
+size_t chol_workspace_bytes(int m);
+int chol_factor_inverse_device(corr_context* c, void* ws, const double* J, int m, double shift,
+                               double* X, double* T, double** Lm_out, bool* ok, void* tc_ws);
 namespace {
 
 __global__ void wait_selftest_kernel(unsigned long long limit_ns, int* status) {
@@ -73,6 +81,40 @@ int corr_selftest_fp64(corr_context* c, int which, long long n, const double* x,
   c->launches += 1;
   CORR_TRY(stage_out(c, out, d_out, (size_t)n * 8));
   return finish_results(c, 0);
+}
+
+int corr_selftest_factor(corr_context* c, int m, const double* J, double* L, double* X) {
+  CORR_CHECK_ARG(c && J && L && X, "corr_selftest_factor: null argument");
+  CORR_CHECK_ARG(m >= 1 && m <= 32768, "corr_selftest_factor: m must be in [1, 32768]");
+  CORR_CUDA(cudaSetDevice(c->device));
+  const size_t nj = (size_t)m * m * 8;
+  auto plan = [&](Carver& w, void** p) {
+    p[0] = w.take(nj);
+    p[1] = w.take(nj);
+    p[2] = w.take(nj);
+    p[3] = w.take(chol_workspace_bytes(m));
+    p[4] = w.take(dgemm_tc_workspace(m, m, m));
+  };
+  void* p[5];
+  Carver cv{nullptr, 0};
+  plan(cv, p);
+  CORR_TRY(c->ws.reserve(cv.used));
+  Carver w{c->ws.ptr, 0};
+  plan(w, p);
+  CORR_CUDA(cudaMemsetAsync(c->dres, 0, sizeof(ResultBlock), c->stream));
+  const double* d_j = static_cast<const double*>(stage_in(c, J, nj, p[0]));
+  CORR_CHECK_ARG(d_j, "host-to-device copy failed");
+  double* d_x = static_cast<double*>(p[1]);
+  double* d_l = nullptr;
+  bool ok = false;
+  CORR_TRY(chol_factor_inverse_device(c, p[3], d_j, m, 0.0, d_x, static_cast<double*>(p[2]), &d_l,
+                                      &ok, p[4]));
+  CORR_TRY(stage_out(c, L, d_l, nj));
+  CORR_TRY(stage_out(c, X, d_x, nj));
+  CORR_TRY(finish_results(c, 0));
+  if (ok) return CORR_OK;
+  set_error("corr_selftest_factor: a pivot is not positive and finite");
+  return CORR_ERR_NOT_PD;
 }
 
 }  // extern "C"

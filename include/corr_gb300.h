@@ -183,6 +183,11 @@ int corr_selftest_wait_timeout(corr_context* ctx, int limit_ms);
  * the FP64 functions that the kernels use in place of the library's. */
 int corr_selftest_fp64(corr_context* ctx, int which, long long n, const double* x, double* out);
 
+/* Diagnostic: the Cholesky factor L of J (m x m, row-major) and X = L^-1, both with
+ * zeros above the diagonal, as the precision forms of corr_rimp2_energy_from_3index
+ * compute them; CORR_ERR_NOT_PD when a pivot is not positive and finite. */
+int corr_selftest_factor(corr_context* ctx, int m, const double* J, double* L, double* X);
+
 /* Tile shape of the tcgen05 energy kernel (no counterpart in the reference).
  * Accepts 0 or 1 and has no effect: every tile runs 128 wide, the padded
  * columns of the last virtual tile being zeros.  (A narrower last tile needs
