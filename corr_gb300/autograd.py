@@ -1,9 +1,10 @@
 """torch.autograd.Function over the GPU RI-MP2 energy and its adjoint.
 
 Forward runs corr_rimp2_energy (FP64 or the tcgen05 precision form); backward
-runs the adjoint of the same form: corr_rimp2_gradient (FP64 panels) after an
-FP64 forward, corr_rimp2_gradient_tc (FP64-accurate digit GEMMs on the tensor
-cores) after a precision-form forward; both recompute the (ia|jb) tiles per
+runs the adjoint of the same form: corr_rimp2_gradient after an FP64 forward
+(FP64-accurate digit GEMMs on the tensor cores, the FP64 pipe in a strict context
+or for values out of their range), corr_rimp2_gradient_tc (the digit GEMMs
+always) after a precision-form forward; both recompute the (ia|jb) panels per
 block of occupied orbitals instead of storing amplitudes.  This module does not import
 psi4, so it can sit next to the syshfwplug plugin without pulling it in.
 """
@@ -36,8 +37,8 @@ class RIMP2Energy(torch.autograd.Function):
     def backward(ctx, gE):
         Bd, ed = ctx.saved_tensors
         nocc, nvir, naux = ctx.dims
-        # the adjoint follows the forward: FP64 panels for the FP64 form, the
-        # tensor-core (digit-GEMM) adjoint for the precision forms
+        # the adjoint follows the forward: for the FP64 form the one that can fall
+        # back to the FP64 pipe, for the precision forms the digit GEMM's
         _, dB, de = ctx.context.rimp2_gradient(Bd, ed, nocc, nvir, naux,
                                                tensor_cores=ctx.precision != "fp64")
         g = gE.to(torch.float64)

@@ -127,7 +127,7 @@ size_t energy_scratch_bytes(corr_context* c, int nocc, int nvir, int naux, int p
 // digit GEMM (panel.cu) rather than the fused FP64 kernel: from (nocc nvir)^2
 // naux = 3e7 on, where the FP64 pipe needs 50 us at its full rate and the
 // panel route's launches about as long (nocc=23 nvir=211 naux=743: 33.2 ms a
-// call against 1.17 ms).
+// call against 1.09 ms).
 bool energy_on_panels(const corr_context* c, int nocc, int nvir, int naux, int precision);
 // host_b (optional): B still in host memory; the precision forms upload it
 // into d_b in row chunks on the context's copy stream, each chunk's row

@@ -49,9 +49,9 @@
 //
 // Bound by the tensor pipe: 36 BF16 products per FP64 product, 53 TFLOP/s at
 // the measured cuBLAS BF16 rate.  Measured, kernel alone: 4096 x 32768 x 2048
-// 10.35 ms (53.1 TFLOP/s; 17.5 ms with four epilogue warps that converted
-// through the FP64 pipe before they released TMEM), 4096 x 4096 x 512 0.376 ms
-// (0.526), 1520^3 0.160 ms (0.266).
+// 10.4 ms (52.6 TFLOP/s; 17.5 ms with four epilogue warps that converted
+// through the FP64 pipe before they released TMEM), 4096 x 4096 x 512 0.344 ms
+// (0.526), 1520^3 0.156 ms (0.266).
 #include <algorithm>
 #include <cmath>
 
@@ -819,7 +819,7 @@ int slice_operand(corr_context* c, const MatView& v, long long r0, int rows, int
 // empty) leave SMs idle, so the tiles of one launch may be split over K.  The
 // cheapest number of parts, counting a K block of 2304 tensor clocks, 3000 for
 // taking a pass's sums out of TMEM, and for split tiles about 6000 more for the
-// exchange through L2.  715^3 (72 tiles): 30 us with two parts, 42 us whole.
+// exchange through L2.  715^3 (72 tiles): 39 us with two parts, 48 us whole.
 constexpr int kSplitSms = 152;
 constexpr int kMaxSplit = 16;
 constexpr long long kMaxSplitSlots = 2 * kSplitSms;

@@ -24,8 +24,9 @@
 //
 // Bound by the FP64 pipe, two FMAs per clock per SM: what counts is FP64
 // instructions per primitive triple, and loads, index arithmetic and local
-// memory run beside them.  20-water cluster: 11.8 ms on the GPU, 13.9 ms a call (25.2 ms with expansions of
-// the auxiliary Gaussians and per-thread E tables).
+// memory run beside them.  20-water cluster: 12.3 ms a call, 2 ms of it the host's
+// screening (25.5 ms with expansions of the auxiliary Gaussians and per-thread E
+// tables).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
