@@ -31,6 +31,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -961,6 +962,9 @@ extern "C" int corr_ri_integrals(corr_context* c, const corr_basis* obs, const c
   }
   CORR_CUDA(cudaMemcpyToSymbolAsync(c_sph, sph, sizeof(sph), 0, cudaMemcpyHostToDevice, c->stream));
   {
+    // built and uploaded once; a second thread's first call waits for that
+    static std::mutex boys_mutex;
+    std::lock_guard<std::mutex> lock(boys_mutex);
     static std::vector<double> boys_tab, boys_exp;
     static bool boys_done[64] = {};
     if (boys_tab.empty()) {
